@@ -30,8 +30,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 BASE_FLAGS = ["-std=c++17", "-O3", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
               "-I" + INCLUDE, "-I" + CSRC] + ARCH
 
-# Non-instantiation sources; gen_generic.cu is compiled once per (dimension, N).
-SOURCES = ["dgop_api.cu", "registry.cu", "basis.cpp", "kron_plan.cpp", "gen_kron3d.cu", "krylov.cu", "host_io.cu", "batch.cu", "batch_solve.cu", "sipdg.cu"]
+# Non-instantiation sources; gen_generic.cu is compiled once per (dimension, N), gen_kronnd.cu per
+# dimension, gen_kron3d.cu per N.
+SOURCES = ["dgop_api.cu", "registry.cu", "basis.cpp", "kron_plan.cpp", "krylov.cu", "host_io.cu", "batch.cu", "batch_solve.cu", "sipdg.cu"]
 
 
 def nvcc():
@@ -76,6 +77,9 @@ def _jobs(fast):
         if not os.path.exists(path):
             raise FileNotFoundError(f"listed source {src} is missing from {CSRC}")
         jobs.append((src, path, []))
+    g3d = os.path.join(CSRC, "gen_kron3d.cu")
+    for n in range(1, 7):
+        jobs.append((f"gen_kron3d_n{n}.cu", g3d, [f"-DDGOP_GEN_N={n}"]))
     gnd = os.path.join(CSRC, "gen_kronnd.cu")
     for d in range(1, 7):
         jobs.append((f"gen_kronnd_d{d}.cu", gnd, [f"-DDGOP_GEN_D={d}"]))

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <deque>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -233,24 +234,68 @@ int setup_launch(dgop_operator* op, LaunchCfg<Real>& L, const Tables1D& t, const
   return DGOP_OK;
 }
 
-// A coefficient in the Kronecker planner's form: a constant, or one product term (no constant).
-SepCoef sep_of(const dgop_coef* c) {
-  SepCoef s;
+// A coefficient as a sum of products (the Kronecker planner's form): its constant and its product
+// terms, where two products that differ along one axis at most (1 and x_2^2, say) become one
+// with the sum of their tables along that axis.  `store` keeps the tables made here.
+std::vector<SepCoef> sep_terms(const dgop_coef* c, const dgop_space& s, int q, std::deque<std::vector<double>>& store,
+                               bool merge) {
+  std::vector<SepCoef> out;
   if (!c) {
-    s.separable = true;
-    s.c = 1.0;
-    return s;
+    out.resize(1);
+    out[0].c = 1.0;
+    out[0].separable = true;
+    return out;
   }
-  s.has_elem = c->element_factor != nullptr;
-  if (c->nterms == 0) {
-    s.separable = true;
-    s.c = c->constant;
-  } else if (c->nterms == 1 && c->constant == 0.0) {
-    s.separable = true;
-    s.c = 1.0;
-    for (int k = 0; k < DGOP_MAX_DIM; ++k) s.tab[k] = c->tables[0][k];
+  if (c->constant != 0.0 || c->nterms == 0) {
+    out.emplace_back();
+    out.back().c = c->constant;
   }
-  return s;
+  for (int t = 0; t < c->nterms; ++t) {
+    out.emplace_back();
+    out.back().c = 1.0;
+    for (int k = 0; k < s.D; ++k) out.back().tab[k] = c->tables[t][k];
+  }
+  auto length = [&](int k) { return (size_t)s.sizes[k] * (q + 2); };
+  auto same = [&](const double* a, const double* b, int k) {
+    return a == b || (a && b && std::memcmp(a, b, sizeof(double) * length(k)) == 0);
+  };
+  for (size_t i = 0; merge && i < out.size(); ++i)
+    for (size_t j = i + 1; j < out.size();) {
+      int differ = -1, count = 0;
+      for (int k = 0; k < s.D; ++k)
+        if (!same(out[i].tab[k], out[j].tab[k], k)) {
+          differ = k;
+          ++count;
+        }
+      if (count > 1) {
+        ++j;
+        continue;
+      }
+      if (count == 0) {
+        out[i].c += out[j].c;
+      } else {
+        std::vector<double> sum(length(differ));
+        for (size_t m = 0; m < sum.size(); ++m)
+          sum[m] = out[i].c * (out[i].tab[differ] ? out[i].tab[differ][m] : 1.0) +
+                   out[j].c * (out[j].tab[differ] ? out[j].tab[differ][m] : 1.0);
+        store.push_back(std::move(sum));
+        out[i].tab[differ] = store.back().data();
+        out[i].c = 1.0;
+      }
+      out.erase(out.begin() + (long)j);
+      j = i + 1;
+    }
+  for (auto& t : out) {
+    t.separable = true;
+    t.has_elem = c->element_factor != nullptr;
+  }
+  return out;
+}
+SepCoef sep_of(const std::vector<SepCoef>& terms) {
+  if (terms.size() == 1) return terms[0];
+  SepCoef none;  // not separable
+  none.has_elem = !terms.empty() && terms[0].has_elem;
+  return none;
 }
 
 // cuTensorMapEncodeTiled, fetched from the driver once (no link against libcuda).
@@ -355,7 +400,9 @@ int launch_kron(const dgop_operator* op, KronCfg<Real>& K, int v, const KronPara
       const int rc = tma_maps_cached(K, T, p.x, p.y, op->sp.nelem);
       if (rc != DGOP_OK) return rc;
       const int tr = (p.flags & kTranspose) ? 1 : 0;
-      T.eflags = K.d_eflags[tr];
+      // per-element factors may have changed since the words were made
+      if (K.factors) K.entry->tma_words(p, K.d_tflags[tr], K.d_gwords[tr], s);
+      T.eflags = K.d_tflags[tr];
       T.gwords = K.d_gwords[tr];
       T.err = K.d_err;
       for (int& m : T.mat_index) m = -1;
@@ -391,12 +438,12 @@ int upload(Real** dst, const double* src, size_t n) {
 
 template <typename Real>
 int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, const double* elem_sigma,
-               const double* const* elem_beta) {
+               const double* const* elem_beta, const double (*face_values)[kMaxN]) {
   const dgop_space& s = op->sp;
   KronEntry<Real>* entry = nullptr;
   if constexpr (sizeof(Real) == 8) entry = &kron3d_slot_f64(s.n);
   else entry = &kron3d_slot_f32(s.n);
-  if (!entry->v[0].launch) {
+  if (!entry->v[1].launch) {
     set_error("no Kronecker kernel for this order");
     return DGOP_ERR_UNSUPPORTED;
   }
@@ -415,13 +462,20 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
   p.has_mass = plan.has_mass;
   p.mass_merged = plan.mass_merged;
   p.g = (Real)op->g;
+  p.general = plan.gl || plan.nextra > 0;
+  p.gl = plan.gl;
+  p.nextra = plan.nextra;
+  for (int f = 0; f < 2; ++f)
+    for (int i = 0; i < s.n; ++i) p.lf[f][i] = (Real)face_values[f][i];
+  for (int t = 0; t < plan.nextra; ++t)
+    for (int k = 0; k < 3; ++k) p.extra[t][k] = plan.extra[t][k];
   int rc = upload<Real>(&K.d_mats, plan.mats.data(), plan.mats.size());
   if (rc) return rc;
   p.mats = K.d_mats;
   // slot -> matrix table; constant tables go to kernel-parameter space
   const int N = s.n;
-  // the kernel reads element-dependent matrices with 16-byte loads when N allows them
-  const int vec = (N % (16 / (int)sizeof(Real)) == 0) ? 16 / (int)sizeof(Real) : 1;
+  // the kernel reads element-dependent matrices with vector loads when N allows them
+  const int vec = kron_vec<Real>(N);
   bool aligned = true;
   auto put = [&](KronParams<Real>& q, int slot, const KronMat& m) {
     q.vary[slot] = 0;
@@ -444,7 +498,7 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     put(p, kSlotTYX, plan.T[1][0]);
     put(p, kSlotTZX, plan.T[2][0]);
     put(p, kSlotTZY, plan.T[2][1]);
-    if (plan.has_mass && !plan.mass_merged) {
+    if (plan.has_mass && !plan.mass_merged && !plan.nextra) {
       put(p, kSlotMD, plan.MD);
       put(p, kSlotMX, plan.MT[0]);
       put(p, kSlotMY, plan.MT[1]);
@@ -468,7 +522,7 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
       p.phi[a] = K.d_phi + phi_off[a];
       for (int k = 0; k < 3; ++k) p.sgn[a][k] = (k == a) ? nullptr : K.d_sgn + sg_off[a][k];
     }
-  } else {
+  } else if (!plan.nextra) {
     put(p, kSlotDZ, plan.MD);
     put(p, kSlotTZX, plan.MT[0]);
     put(p, kSlotTZY, plan.MT[1]);
@@ -496,6 +550,8 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     put(K.params_t, kSlotDY, plan.Dt[1]);
     put(K.params_t, kSlotDZ, plan.Dt[2]);
   }
+  for (int t = 0; t < plan.nextra; ++t)
+    for (int k = 0; k < 3; ++k) aligned = aligned && plan.extra[t][k].off % vec == 0 && plan.extra[t][k].stride % vec == 0;
   if (!aligned) {
     set_error("Kronecker matrix table misaligned for vector loads");
     return DGOP_ERR_UNSUPPORTED;
@@ -504,24 +560,45 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
   // shape per kernel variant (their shared memory per warp differs)
   int max_smem = 0;
   DGOP_CUDA(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, op->device));
-  const bool sep = plan.has_adv && plan.has_mass && !plan.mass_merged;
+  const bool sep = plan.has_adv && plan.has_mass && !plan.mass_merged && !plan.nextra;
   const int64_t groups = (s.nelem + entry->epw - 1) / entry->epw;
   // bulk-tensor variants: groups of 8 elements inside one x-row, plane rows addressable by int
-  const bool tma_shape = entry->face_words && s.sizes[0] % 8 == 0 && s.nelem % 8 == 0 &&
+  const bool tma_shape = entry->tma_words && !p.general && s.sizes[0] % 8 == 0 && s.nelem % 8 == 0 &&
                          s.nelem < (int64_t(1) << 29) && tensor_map_encoder() != nullptr;
-  if (tma_shape) {
-    for (int tr = 0; tr < 2; ++tr) {
-      DGOP_CUDA(cudaMalloc(&K.d_eflags[tr], sizeof(uint32_t) * s.nelem));
-      DGOP_CUDA(cudaMalloc(&K.d_gwords[tr], sizeof(uint32_t) * (s.nelem / 8)));
-      KronParams<Real> q = tr ? K.params_t : p;
-      q.flags = op->flags | (tr ? kTranspose : 0);
-      entry->face_words(q, K.d_eflags[tr], K.d_gwords[tr], 0);
+  // face words, unless per-element velocity factors decide the faces anew in every apply: made once
+  // for both precisions (the signs that decide are the FP64 ones)
+  for (int a = 0; a < 3; ++a) K.factors = K.factors || p.elem[a];
+  KronParams<Real> fw = p, tr = K.params_t;
+  fw.flags = op->flags;
+  tr.flags = op->flags | kTranspose;
+  bool wait = false;
+  if (plan.has_adv && !K.factors) {
+    if (!op->d_face_words) {
+      DGOP_CUDA(cudaMalloc(&op->d_face_words, 2 * sizeof(uint32_t) * s.nelem));
+      entry->face_words(fw, tr, op->d_face_words, 0);
       DGOP_CUDA(cudaGetLastError());
+      wait = true;
     }
-    DGOP_CUDA(cudaMalloc(&K.d_err, sizeof(int)));
-    DGOP_CUDA(cudaMemset(K.d_err, 0, sizeof(int)));
-    DGOP_CUDA(cudaDeviceSynchronize());
+    p.eflags = op->d_face_words;
+    K.params_t.eflags = op->d_face_words + s.nelem;
   }
+  if (tma_shape) {
+    // one allocation: face words and slot words, forward and transposed, then the error word
+    const size_t nw = (size_t)s.nelem, ng = (size_t)s.nelem / 8;
+    DGOP_CUDA(cudaMalloc(&K.d_tma, sizeof(uint32_t) * (2 * (nw + ng) + 1)));
+    K.d_tflags[0] = K.d_tma;
+    K.d_tflags[1] = K.d_tma + nw;
+    K.d_gwords[0] = K.d_tma + 2 * nw;
+    K.d_gwords[1] = K.d_tma + 2 * nw + ng;
+    K.d_err = reinterpret_cast<int*>(K.d_tma + 2 * (nw + ng));
+    DGOP_CUDA(cudaMemset(K.d_err, 0, sizeof(int)));
+    entry->tma_words(fw, K.d_tflags[0], K.d_gwords[0], 0);
+    entry->tma_words(tr, K.d_tflags[1], K.d_gwords[1], 0);
+    DGOP_CUDA(cudaGetLastError());
+    wait = true;
+  }
+  // applies may come on any stream: the words are ready before the operator is returned
+  if (wait) DGOP_CUDA(cudaDeviceSynchronize());
   int usable = 0;
   for (int v = 0; v < kKronVariants; ++v) {
     const KronVariant<Real>& kv = entry->v[v];
@@ -536,6 +613,9 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     if (arc == DGOP_OK) arc = allow_dynamic_smem(kv.func_sep, max_smem);
     for (const void* f : kv.func_dot)
       if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
+    for (const auto& by_sep : kv.func_general)
+      for (const void* f : by_sep)
+        if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
     for (const auto& by_dot : kv.func_masked)
       for (const auto& by_sep : by_dot)
         for (const void* f : by_sep)
@@ -546,7 +626,8 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     const int mi = kron_mask_index(p);
     const void* kern[2] = {sep ? kv.func_sep : kv.func, kv.func_dot[sep ? 1 : 0]};
     for (int dot = 0; dot < 2; ++dot)
-      if (mi >= 0 && kv.func_masked[mi][dot][sep ? 1 : 0]) kern[dot] = kv.func_masked[mi][dot][sep ? 1 : 0];
+      if (p.general) kern[dot] = kv.func_general[dot][sep ? 1 : 0];
+      else if (mi >= 0 && kv.func_masked[mi][dot][sep ? 1 : 0]) kern[dot] = kv.func_masked[mi][dot][sep ? 1 : 0];
     int per_sm = 0, per_sm_dot = 0;
     DGOP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[0], threads, L.smem));
     if (per_sm < 1) continue;
@@ -1071,11 +1152,7 @@ void free_kronnd(KronNDCfg<Real>& K) {
 
 template <typename Real>
 void free_kron(KronCfg<Real>& K) {
-  for (int tr = 0; tr < 2; ++tr) {
-    if (K.d_eflags[tr]) cudaFree(K.d_eflags[tr]);
-    if (K.d_gwords[tr]) cudaFree(K.d_gwords[tr]);
-  }
-  if (K.d_err) cudaFree(K.d_err);
+  if (K.d_tma) cudaFree(K.d_tma);
   if (K.d_mats) cudaFree(K.d_mats);
   if (K.d_phi) cudaFree(K.d_phi);
   if (K.d_sgn) cudaFree(K.d_sgn);
@@ -1171,12 +1248,17 @@ int create_operator(const dgop_space* space, int q, const dgop_coef* sigma, cons
     in.Dq = t.Dq;
     in.wq = t.wq;
     const dgop_coef* sg = (flags & kMass) ? (sigma ? sigma : &one) : nullptr;
-    in.sigma = sep_of(sg);
+    // (the mass inverse takes a single product as the caller gave it)
+    std::deque<std::vector<double>> store;
+    const std::vector<SepCoef> sigma_terms = sep_terms(sg, op->sp, q, store, !(flags & kInvMass));
+    in.sigma = sep_of(sigma_terms);
+    in.sigma_terms = sigma_terms.data();
+    in.num_sigma_terms = (int)sigma_terms.size();
     in.inverse_mass = (flags & kInvMass) != 0;
     const bool adv = (flags & (kAdvCell | kFaceInt | kFaceBnd)) != 0;
     const double* elem_beta[kMaxDim] = {};
     for (int k = 0; k < op->sp.D; ++k) {
-      in.beta[k] = sep_of(adv ? &beta[k] : nullptr);
+      in.beta[k] = sep_of(sep_terms(adv ? &beta[k] : nullptr, op->sp, q, store, true));
       elem_beta[k] = adv ? beta[k].element_factor : nullptr;
     }
     // any-dimension kernel: every shape the Kronecker form covers (also the 3D register kernel's,
@@ -1195,9 +1277,9 @@ int create_operator(const dgop_space* space, int q, const dgop_coef* sigma, cons
     KronPlanHost plan = plan_kron3d(in);
     if (plan.ok) {
       const double* es = sg ? sg->element_factor : nullptr;
-      const int krc = setup_kron<double>(op, op->k64, plan, es, elem_beta);
+      const int krc = setup_kron<double>(op, op->k64, plan, es, elem_beta, t.Bf);
       if (krc == DGOP_OK) {
-        if (setup_kron<float>(op, op->k32, plan, es, elem_beta) != DGOP_OK) free_kron(op->k32);
+        if (setup_kron<float>(op, op->k32, plan, es, elem_beta, t.Bf) != DGOP_OK) free_kron(op->k32);
         op->kernel = DGOP_KERNEL_KRON;
         autotune_kron(op, op->k64);
         autotune_kron(op, op->k32);
@@ -1218,6 +1300,7 @@ int create_operator(const dgop_space* space, int q, const dgop_coef* sigma, cons
     free_launch(op->f32);
     free_kron(op->k32);
     free_kronnd(op->n32);
+    if (op->d_face_words) cudaFree(op->d_face_words);
     delete op;
     set_error(generic_err.empty() ? std::string("no kernel for this operator") : generic_err);
     return DGOP_ERR_UNSUPPORTED;
@@ -1606,6 +1689,7 @@ int dgop_operator_destroy(dgop_operator* op) {
   free_kronnd(op->n32);
   free_diff(op->s64);
   free_diff(op->s32);
+  if (op->d_face_words) cudaFree(op->d_face_words);
   delete op;
   return DGOP_OK;
 }

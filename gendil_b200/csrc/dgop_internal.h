@@ -54,9 +54,12 @@ struct KronCfg {
   Real* d_phi = nullptr;
   signed char* d_sgn = nullptr;
   Real* d_elem[4] = {};  // converted per-element factors (FP32 only)
-  // bulk-tensor variants: face words per element and slot words per group of 8 elements, for
-  // the forward [0] and transposed [1] operator; a device word set when a bounded wait gives up
-  uint32_t* d_eflags[2] = {};
+  bool factors = false;  // per-element velocity factors
+  // bulk-tensor variants: face words per element and slot words per group of 8 elements, for the
+  // forward [0] and transposed [1] operator, and a device word set when a bounded wait gives up,
+  // all in d_tma
+  uint32_t* d_tma = nullptr;
+  uint32_t* d_tflags[2] = {};
   uint32_t* d_gwords[2] = {};
   int* d_err = nullptr;
   // tensor maps of recent (x, y) pairs (opaque CUtensorMap bytes: group, z slices, y slices,
@@ -134,6 +137,7 @@ struct dgop_operator {
   dgop::LaunchCfg<float> f32;
   dgop::KronCfg<double> k64;
   dgop::KronCfg<float> k32;
+  uint32_t* d_face_words = nullptr;  // 3D register kernel: face words, forward then transposed
   dgop::KronNDCfg<double> n64;
   dgop::KronNDCfg<float> n32;
   dgop::KronDiffCfg<double> s64;  // interior-penalty diffusion (dgop_sipdg_create)

@@ -1,44 +1,48 @@
-// Instantiations of the 3D Kronecker-form kernel, N = 1..5, FP64 and FP32, every variant.
+// Instantiations of the 3D Kronecker-form kernel, FP64 and FP32, every variant; compiled once per
+// order with -DDGOP_GEN_N=<p + 1>, N = 1..6.
 #include "kron3d_kernel.cuh"
 #include "kron3d_tma_kernel.cuh"
 #include "kron_registry.h"
 
+#include <algorithm>
 #include <type_traits>
+
+#ifndef DGOP_GEN_N
+#error "DGOP_GEN_N must be defined"
+#endif
+#define DGOP_CAT2_(a, b) a##b
+#define DGOP_CAT2(a, b) DGOP_CAT2_(a, b)
 
 namespace dgop {
 
+#if DGOP_GEN_N == 1
 const char* const kKronVariantNames[kKronVariants] = {"stage2-tile", "stage1-tile", "stage2-shfl",
                                                       "tma1-tile",   "tma2-shfl",   "tma2-tile"};
 // (the any-dimension kernel's variants, kronnd_kernel.cuh, named here with the 3D kernel's)
 const char* const kKronNDVariantNames[kKronNDVariants] = {"nd-passes", "nd-grouped2", "nd-grouped3", "nd-paired",
                                                           "nd-mass"};
+#endif
 
 namespace {
-// The one-stage tile variant at N = 4 (p = 3) is also compiled for the masks kVaryNone and
+// The one-stage tile variant at N >= 4 (p >= 3) is also compiled for the masks kVaryNone and
 // kVarySheared; an operator whose mask is exactly one of them runs that kernel, every other
 // operator the run-time-mask kernel (same arithmetic, same results).
+template <int N, int STAGES, bool SHFL>
+constexpr bool masked_forms() {
+  return N >= 4 && STAGES == 1 && !SHFL;
+}
+
 template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT>
 void launch_kron3d_masked(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
-  if constexpr (N == 4 && STAGES == 1 && !SHFL) {
+  if constexpr (masked_forms<N, STAGES, SHFL>()) {
     const int mi = kron_mask_index(p);
-    if constexpr (std::is_same<Real, double>::value && !SEP) {
-      if (mi == 0) {
-        kron3d_kernel_capped<N, STAGES, SHFL, DOT, kVaryNone><<<grid, block, smem, s>>>(p);
-        return;
-      }
-      if (mi == 1) {
-        kron3d_kernel_capped<N, STAGES, SHFL, DOT, kVarySheared><<<grid, block, smem, s>>>(p);
-        return;
-      }
-    } else {
-      if (mi == 0) {
-        kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, kVaryNone><<<grid, block, smem, s>>>(p);
-        return;
-      }
-      if (mi == 1) {
-        kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, kVarySheared><<<grid, block, smem, s>>>(p);
-        return;
-      }
+    if (mi == 0) {
+      kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, kVaryNone><<<grid, block, smem, s>>>(p);
+      return;
+    }
+    if (mi == 1) {
+      kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, kVarySheared><<<grid, block, smem, s>>>(p);
+      return;
     }
   }
   kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT><<<grid, block, smem, s>>>(p);
@@ -46,7 +50,19 @@ void launch_kron3d_masked(const KronParams<Real>& p, dim3 grid, dim3 block, size
 
 template <int N, typename Real, int STAGES, bool SHFL>
 void launch_kron3d(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
-  const bool sep = p.has_adv && p.has_mass && !p.mass_merged;
+  const bool sep = p.has_adv && p.has_mass && !p.mass_merged && !p.nextra;
+  if (p.general) {
+    if constexpr (std::is_same<Real, double>::value) {
+      if (p.dot_partials) {
+        if (sep) kron3d_kernel<N, Real, true, STAGES, SHFL, true, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
+        else kron3d_kernel<N, Real, false, STAGES, SHFL, true, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
+        return;
+      }
+    }
+    if (sep) kron3d_kernel<N, Real, true, STAGES, SHFL, false, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
+    else kron3d_kernel<N, Real, false, STAGES, SHFL, false, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
+    return;
+  }
   if constexpr (std::is_same<Real, double>::value) {
     if (p.dot_partials) {
       if (sep) launch_kron3d_masked<N, Real, true, STAGES, SHFL, true>(p, grid, block, smem, s);
@@ -58,39 +74,43 @@ void launch_kron3d(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem
   else launch_kron3d_masked<N, Real, false, STAGES, SHFL, false>(p, grid, block, smem, s);
 }
 
+template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false>
+const void* kernel_of() {
+  return reinterpret_cast<const void*>(&kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>);
+}
+
 template <int N, typename Real, int STAGES, bool SHFL>
 void fill_variant(KronVariant<Real>& v) {
   v.launch = &launch_kron3d<N, Real, STAGES, SHFL>;
-  v.func = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, false, STAGES, SHFL>);
-  v.func_sep = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, true, STAGES, SHFL>);
+  v.func = kernel_of<N, Real, STAGES, SHFL, false, false, kVaryRuntime>();
+  v.func_sep = kernel_of<N, Real, STAGES, SHFL, true, false, kVaryRuntime>();
   if constexpr (std::is_same<Real, double>::value) {
-    v.func_dot[0] = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, false, STAGES, SHFL, true>);
-    v.func_dot[1] = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, true, STAGES, SHFL, true>);
+    v.func_dot[0] = kernel_of<N, Real, STAGES, SHFL, false, true, kVaryRuntime>();
+    v.func_dot[1] = kernel_of<N, Real, STAGES, SHFL, true, true, kVaryRuntime>();
   }
-  if constexpr (N == 4 && STAGES == 1 && !SHFL) {
-    v.func_masked[0][0][1] = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, true, 1, false, false, kVaryNone>);
-    v.func_masked[1][0][1] = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, true, 1, false, false, kVarySheared>);
+  if constexpr (masked_forms<N, STAGES, SHFL>()) {
+    v.func_masked[0][0][0] = kernel_of<N, Real, STAGES, SHFL, false, false, kVaryNone>();
+    v.func_masked[0][0][1] = kernel_of<N, Real, STAGES, SHFL, true, false, kVaryNone>();
+    v.func_masked[1][0][0] = kernel_of<N, Real, STAGES, SHFL, false, false, kVarySheared>();
+    v.func_masked[1][0][1] = kernel_of<N, Real, STAGES, SHFL, true, false, kVarySheared>();
     if constexpr (std::is_same<Real, double>::value) {
-      v.func_masked[0][0][0] = reinterpret_cast<const void*>(&kron3d_kernel_capped<N, 1, false, false, kVaryNone>);
-      v.func_masked[1][0][0] = reinterpret_cast<const void*>(&kron3d_kernel_capped<N, 1, false, false, kVarySheared>);
-      v.func_masked[0][1][0] = reinterpret_cast<const void*>(&kron3d_kernel_capped<N, 1, false, true, kVaryNone>);
-      v.func_masked[1][1][0] = reinterpret_cast<const void*>(&kron3d_kernel_capped<N, 1, false, true, kVarySheared>);
-      v.func_masked[0][1][1] = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, true, 1, false, true, kVaryNone>);
-      v.func_masked[1][1][1] =
-          reinterpret_cast<const void*>(&kron3d_kernel<N, Real, true, 1, false, true, kVarySheared>);
-    } else {
-      v.func_masked[0][0][0] = reinterpret_cast<const void*>(&kron3d_kernel<N, Real, false, 1, false, false, kVaryNone>);
-      v.func_masked[1][0][0] =
-          reinterpret_cast<const void*>(&kron3d_kernel<N, Real, false, 1, false, false, kVarySheared>);
+      v.func_masked[0][1][0] = kernel_of<N, Real, STAGES, SHFL, false, true, kVaryNone>();
+      v.func_masked[0][1][1] = kernel_of<N, Real, STAGES, SHFL, true, true, kVaryNone>();
+      v.func_masked[1][1][0] = kernel_of<N, Real, STAGES, SHFL, false, true, kVarySheared>();
+      v.func_masked[1][1][1] = kernel_of<N, Real, STAGES, SHFL, true, true, kVarySheared>();
     }
+  }
+  v.func_general[0][0] = kernel_of<N, Real, STAGES, SHFL, false, false, kVaryRuntime, true>();
+  v.func_general[0][1] = kernel_of<N, Real, STAGES, SHFL, true, false, kVaryRuntime, true>();
+  if constexpr (std::is_same<Real, double>::value) {
+    v.func_general[1][0] = kernel_of<N, Real, STAGES, SHFL, false, true, kVaryRuntime, true>();
+    v.func_general[1][1] = kernel_of<N, Real, STAGES, SHFL, true, true, kVaryRuntime, true>();
   }
   v.warp_smem = Kron3DShape<N, Real>::warp_smem(STAGES, SHFL);
   v.threads = kKronThreads;
 }
 
-// The one-stage tile variant (the fastest on the 3D p=3 workloads) is also compiled for the
-// masks kVaryNone and kVarySheared (kron.h); an operator whose mask is exactly one of them runs
-// that kernel, every other operator the run-time-mask kernel (same arithmetic, same results).
+// (the bulk-tensor one-stage tile variant has the same compiled masks)
 template <bool SEP, int STAGES, bool SHFL, bool DOT>
 void launch_tma_masked(const KronTmaParams<double>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
   if constexpr (STAGES == 1 && !SHFL) {
@@ -141,39 +161,39 @@ void fill_tma(KronVariant<double>& v) {
 }
 
 template <typename Real>
-void face_words(const KronParams<Real>& p, uint32_t* eflags, uint32_t* gwords, cudaStream_t s) {
+void face_words(const KronParams<Real>& fwd, const KronParams<Real>& tr, uint32_t* words, cudaStream_t s) {
+  const int64_t blocks = std::min<int64_t>((fwd.nelem + 255) / 256, 4096);
+  kron_face_words<Real><<<(unsigned)blocks, 256, 0, s>>>(fwd, tr, words);
+}
+template <typename Real>
+void tma_words(const KronParams<Real>& p, uint32_t* eflags, uint32_t* gwords, cudaStream_t s) {
   const int64_t groups = (p.nelem + 7) / 8;
   const int64_t blocks = (groups * 32 + 255) / 256;
-  kron_face_words<Real><<<(unsigned)blocks, 256, 0, s>>>(p, eflags, gwords);
+  kron_tma_words<Real><<<(unsigned)blocks, 256, 0, s>>>(p, eflags, gwords);
 }
 
 template <int N, typename Real>
 void fill(KronEntry<Real>& d) {
   d.epw = Kron3DShape<N, Real>::EPW;
-  fill_variant<N, Real, 2, false>(d.v[0]);
+  // above p = 3 one staging stage: two of them and the exchange tile leave too few warps per SM
+  if constexpr (N <= 4) fill_variant<N, Real, 2, false>(d.v[0]);
   fill_variant<N, Real, 1, false>(d.v[1]);
   if constexpr (Kron3DShape<N, Real>::BUTTERFLY) fill_variant<N, Real, 2, true>(d.v[2]);
-  if constexpr (N == 4 && std::is_same<Real, double>::value) {
+  d.face_words = &face_words<Real>;
+#if DGOP_GEN_N == 4
+  if constexpr (std::is_same<Real, double>::value) {
     fill_tma<1, false>(d.v[3]);
     fill_tma<2, true>(d.v[4]);
     fill_tma<2, false>(d.v[5]);
-    d.face_words = &face_words<Real>;
+    d.tma_words = &tma_words<Real>;
   }
-}
-
-template <int N>
-void reg_one() {
-  fill<N, double>(kron3d_slot_f64(N));
-  fill<N, float>(kron3d_slot_f32(N));
+#endif
 }
 }  // namespace
 
-void register_kron3d() {
-  reg_one<1>();
-  reg_one<2>();
-  reg_one<3>();
-  reg_one<4>();
-  reg_one<5>();
+void DGOP_CAT2(register_kron3d_n, DGOP_GEN_N)() {
+  fill<DGOP_GEN_N, double>(kron3d_slot_f64(DGOP_GEN_N));
+  fill<DGOP_GEN_N, float>(kron3d_slot_f32(DGOP_GEN_N));
 }
 
 }  // namespace dgop

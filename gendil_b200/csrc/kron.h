@@ -27,7 +27,9 @@
 
 namespace dgop {
 
-constexpr int kKronMaxN = 5;
+constexpr int kKronMaxN = 6;  // largest order of the 3D register kernel, plus one
+
+constexpr int kKronMaxExtra = kMaxTerms + 1;  // mass terms of a density: a constant and its products
 
 // A per-axis matrix table: matrix for element coordinate e at off + e * stride (stride 0: one
 // matrix for all elements).  Offsets are into the plan's matrix buffer.
@@ -53,6 +55,12 @@ enum KronSlot : int {
   kNumSlots = 12
 };
 
+// Values per vector access of the 3D kernel's planes and matrix rows: 16 bytes when N allows it.
+template <typename Real>
+constexpr int kron_vec(int N) {
+  return N % (16 / (int)sizeof(Real)) == 0 ? 16 / (int)sizeof(Real) : (sizeof(Real) == 4 && N % 2 == 0 ? 2 : 1);
+}
+
 template <typename Real>
 struct KronParams {
   int64_t nelem;      // < 2^32 (checked by the planner); the launch processes [e_begin, nelem)
@@ -76,6 +84,12 @@ struct KronParams {
   const signed char* sgn[3][3];  // sgn[a][k][e_k] in {-1, 0, 1} (k != a)
   const Real* elem[3];           // per-element beta_a factor or nullptr
   const Real* elem_mass;         // per-element sigma factor or nullptr
+  // general form (kron3d_kernel.cuh): a basis without nodes on the faces (lf: its values there),
+  // and mass terms extra[t] = matrices along x, y, z (a density that is a sum of products)
+  int general, gl, nextra;
+  Real lf[2][kKronMaxN];
+  KronMat extra[kKronMaxExtra][3];
+  const uint32_t* eflags;        // face word per element (kron3d_kernel.cuh); null: built in the kernel
   const int* skip;               // device word; the launch does nothing when it is non-zero
   // optional epilogue: dot_partials[b] = sum over CTA b's outputs of dot_z . y (fixed order),
   // entries b >= gridDim.x of the first dot_count zeroed (dot_partials null: no epilogue)
@@ -190,6 +204,10 @@ struct KronPlanHost {
   // the last axis, MT[k] along the others
   KronMat D[kMaxDim], Dt[kMaxDim], T[kMaxDim][kMaxDim], MD, MT[kMaxDim];
   int has_adv = 0, has_mass = 0, mass_merged = 0;
+  // general form (3D): basis values at the two faces, mass terms of a sum of products
+  bool gl = false;
+  int nextra = 0;
+  KronMat extra[kKronMaxExtra][kMaxDim];
 };
 
 // Host-side description of one scalar coefficient: c * prod_k table_k (table_k may be null).

@@ -1,26 +1,31 @@
-// Register-resident Kronecker-form DG operator kernel for 3D hexahedra, N = p + 1 <= 5.
+// Register-resident Kronecker-form DG operator kernel for 3D hexahedra, N = p + 1 <= 6.
 //
 // N consecutive lanes own one element; lane t holds an N x N plane of it in registers:
 //   layout Z: plane z = t, values [x][y]      layout Y: plane y = t, values [x][z]
-// Operators along x and y run in layout Z, along x and z in layout Y.  Schedule per element
-// (9 n x n passes, 4 layout exchanges):
+// Every term (x)_k A_k is a plane phase (its x and y factors, in place, in layout Z), one exchange
+// to layout Y and its z factor, accumulated there:
 //
-//   Z: px = Dx u + x-faces ; qx = Txy px ; py = Dy u + y-faces             exchange qx, py -> Y
-//   Y: out = Txz qx + Tyx Tyz py ; pz = Dz u + z-faces (mass merged) ; qz = Tzx pz
-//                                                                           exchange qz, out -> Z
-//   Z: out += Tzy qz ; y = alpha out + beta y
+//   x term: Dx, x faces, Txy                | exchange |  out  = Txz .
+//   y term: Dy, y faces, Tyx                | exchange |  out += Tyz .
+//   z term: Tzx, Tzy                        | exchange |  out += Dz . + z faces   (mass merged in Dz)
+//   a separate mass term: Mx, My            | exchange |  out += Md .
 //
-// The upwind neighbour trace of every inflow face is added to the face slice of the D-pass
-// output, so the tangential passes that follow apply the face's tangential operator to it.
+// Three exchanges and one plane live beside the accumulator (the order x, z, y with the faces at
+// each term's start needs four exchanges and two more planes).  The upwind neighbour trace of an
+// inflow face is added to the face slice of the D-pass output, so the tangential passes that
+// follow apply the face's tangential operator to it; the z faces come after the tangential
+// passes, so the z neighbours' slices pass through Tzy and Tzx on their own: lane t takes column
+// x = t through Tzy, then row y = t through Tzx (2 N^2 multiply-adds per lane against 9 N^3).
 //
 // Memory: each warp loops over groups of 32/N consecutive elements (persistent grid).  The
-// group's DoFs, the neighbour traces its inflow faces need and a per-element record of its face
-// decisions are staged into padded shared memory one group ahead (double buffered, coalesced
-// cp.async copies), so loads of the next group overlap the arithmetic of this one; results leave
-// through the same buffer with coalesced stores.  Constant 1D matrices are read from
-// kernel-parameter space, only element-dependent ones from global memory.  For even N the layout
-// exchanges are register butterflies (shfl_xor within the element's lanes); odd N exchange
-// through a shared tile.
+// group's DoFs and the neighbour traces its inflow faces need are staged into padded shared
+// memory (coalesced cp.async copies; STAGES = 2: one group ahead), each term reads its plane from
+// there, and results leave through the same buffer with coalesced stores.  Which traces an element
+// needs is one 32-bit face word per element, built at operator creation (kron_face_words); with
+// per-element velocity factors, which the caller may change between applies, the word is built
+// in the kernel.  Constant 1D matrices are read from kernel-parameter space, only
+// element-dependent ones from global memory.  For even N the layout exchanges can be register
+// butterflies (shfl_xor within the element's lanes); otherwise they go through a shared tile.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -41,7 +46,7 @@ struct Kron3DShape {
   static constexpr int CR = CB / (int)sizeof(Real);  // Reals per chunk
   static constexpr int pad_for(int p) { return ((NN + p) * (int)sizeof(Real)) % CB == 0 ? p : pad_for(p + 1); }
   // vector width (Reals) of shared-memory accesses along x: 16 bytes when N allows it
-  static constexpr int V = (N % (16 / (int)sizeof(Real)) == 0) ? 16 / (int)sizeof(Real) : 1;
+  static constexpr int V = kron_vec<Real>(N);
   // Shared-memory bank model: accesses of G bytes are served 128 bytes at a time (8, 16 or 32
   // lanes together); two lanes of one such phase conflict when their G-byte granules fall in the
   // same bank group.  `distinct` checks one access pattern: offset(le, t) in Reals.
@@ -85,23 +90,23 @@ struct Kron3DShape {
   }
   static constexpr int SP = staged_geom().SP;  // staged plane stride (Reals)
   static constexpr int SE = staged_geom().SE;  // staged element stride
-  // neighbour traces: one slot per axis (N rows of N), used by the first face of that axis that
-  // needs a neighbour trace; a second one on the same axis (rare) is read from global memory.
+  // neighbour traces (N rows of N values): slots 0 and 1 for the first x and y face that needs a
+  // neighbour's trace (a second one on the same axis, rare, is read from global memory), slots 2
+  // and 3 for the two z faces (their traces pass through the tangential factors in place).
   // Rows are read V-wide; the element stride TE is the smallest conflict-free one.
   static constexpr int RB = (N * (int)sizeof(Real)) % 16 == 0 ? 16 : ((N * (int)sizeof(Real)) % 8 == 0 ? 8 : 4);
   static constexpr int TR = N;                // trace row stride
   static constexpr int TS = N * TR;           // trace slot stride
+  static constexpr int kTraceSlots = 4;
   static constexpr int trace_stride() {
-    for (int te = 3 * TS; te <= 3 * TS + 64; ++te) {
+    for (int te = kTraceSlots * TS; te <= kTraceSlots * TS + 64; ++te) {
       if ((te * (int)sizeof(Real)) % RB || te % V) continue;
       if (distinct(V, [&](int le, int t) { return le * te + t * TR; })) return te;
     }
-    return 3 * TS;
+    return kTraceSlots * TS;
   }
   static constexpr int TE = trace_stride();   // traces per element
-  // face record per element: 12 coefficients (axis, side, {corner, neighbour/inflow}) + flag word
-  static constexpr int RE = 12 + (16 / (int)sizeof(Real));
-  static constexpr int STAGE = EPW * (SE + TE + RE);  // one pipeline stage: DoFs, traces, records
+  static constexpr int STAGE = (EPW * (SE + TE) + 3) / 4 * 4;  // one pipeline stage: DoFs, traces
   static constexpr bool BUTTERFLY = (N == 2 || N == 4);  // shuffle exchanges possible
   // Exchange tile per element, layout [y][z][x]: value (x, y, z) at y * TA + z * N + x, element
   // stride TSE.  Both sides of an exchange access V consecutive x values; TA and TSE are the
@@ -212,34 +217,6 @@ __device__ __forceinline__ void vldg(const Real* p, Real (&v)[V]) {
   }
 }
 
-// Y[i][j] = sum_r A(i, r) X[r][j]      (operator along the first plane index)
-template <int N, typename Real, typename Mat>
-__device__ __forceinline__ void apply_first(const Mat& A, const Real (&X)[N][N], Real (&Y)[N][N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      Real s = A(i, 0) * X[0][j];
-#pragma unroll
-      for (int r = 1; r < N; ++r) s += A(i, r) * X[r][j];
-      Y[i][j] = s;
-    }
-}
-
-// Y[i][j] = sum_r A(j, r) X[i][r]      (operator along the second plane index)
-template <int N, typename Real, typename Mat>
-__device__ __forceinline__ void apply_second(const Mat& A, const Real (&X)[N][N], Real (&Y)[N][N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      Real s = A(j, 0) * X[i][0];
-#pragma unroll
-      for (int r = 1; r < N; ++r) s += A(j, r) * X[i][r];
-      Y[i][j] = s;
-    }
-}
-
 template <int N, typename Real>
 struct RegMat {
   Real a[N][N];
@@ -252,36 +229,191 @@ struct ParamMat {
   __device__ __forceinline__ Real operator()(int i, int j) const { return P.cm[SLOT][i * N + j]; }
 };
 
-// Apply slot SLOT's matrix (for element coordinate `coord` along its axis) along the first or
-// second plane index: constant matrices come from kernel-parameter space.  VM: the slot mask the
-// kernel is compiled for (kron.h).
-template <int N, typename Real, int SLOT, bool FIRST, uint32_t VM = kVaryRuntime>
-__device__ __forceinline__ void kron_apply(const KronParams<Real>& P, uint32_t coord, const Real (&X)[N][N],
-                                           Real (&Y)[N][N]) {
-  bool vary;
-  if constexpr (VM == kVaryRuntime) vary = P.vary[SLOT] != 0;
-  else vary = ((VM >> SLOT) & 1u) != 0;
-  if (vary) {
-    RegMat<N, Real> A;
-    const Real* p = P.mats + P.vm[SLOT].off + (int64_t)coord * P.vm[SLOT].stride;
-    // N x N blocks at offsets that are multiples of the vector width (checked at setup)
-    constexpr int V = Kron3DShape<N, Real>::V;
+// Whether slot SLOT's matrix depends on the element: from the slot mask the kernel is compiled
+// for (kron.h), or at run time.
+template <int SLOT, uint32_t VM, typename Real>
+__device__ __forceinline__ bool slot_varies(const KronParams<Real>& P) {
+  if constexpr (VM == kVaryRuntime) return P.vary[SLOT] != 0;
+  else return ((VM >> SLOT) & 1u) != 0;
+}
+// Slot SLOT's matrix for element coordinate `coord` along its axis (element-dependent slots).
+template <int SLOT, typename Real>
+__device__ __forceinline__ const Real* slot_matrix(const KronParams<Real>& P, uint32_t coord) {
+  return P.mats + P.vm[SLOT].off + (int64_t)coord * P.vm[SLOT].stride;
+}
+
+// Row i of an N x N matrix at p (16-byte aligned when V > 1).
+template <int N, typename Real>
+__device__ __forceinline__ void matrix_row(const Real* p, int i, Real (&row)[N]) {
+  constexpr int V = Kron3DShape<N, Real>::V;
 #pragma unroll
-    for (int i = 0; i < N; ++i)
+  for (int j = 0; j < N; j += V) {
+    Real v[V];
+    vldg<Real, V>(p + i * N + j, v);
 #pragma unroll
-      for (int j = 0; j < N; j += V) {
-        Real v[V];
-        vldg<Real, V>(p + i * N + j, v);
-#pragma unroll
-        for (int q = 0; q < V; ++q) A.a[i][j + q] = v[q];
-      }
-    if (FIRST) apply_first<N>(A, X, Y);
-    else apply_second<N>(A, X, Y);
-  } else {
-    ParamMat<N, Real, SLOT> A{P};
-    if (FIRST) apply_first<N>(A, X, Y);
-    else apply_second<N>(A, X, Y);
+    for (int q = 0; q < V; ++q) row[j + q] = v[q];
   }
+}
+template <int N, typename Real>
+__device__ __forceinline__ void load_matrix(const Real* p, RegMat<N, Real>& A) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) matrix_row<N>(p, i, A.a[i]);
+}
+
+// X <- A X along the first (FIRST) or second plane index, line by line.
+template <int N, bool FIRST, typename Real, typename Mat>
+__device__ __forceinline__ void lines_inplace(const Mat& A, Real (&X)[N][N]) {
+#pragma unroll
+  for (int l = 0; l < N; ++l) {
+    Real w[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      Real s = A(j, 0) * (FIRST ? X[0][l] : X[l][0]);
+#pragma unroll
+      for (int i = 1; i < N; ++i) s += A(j, i) * (FIRST ? X[i][l] : X[l][i]);
+      w[j] = s;
+    }
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if constexpr (FIRST) X[j][l] = w[j];
+      else X[l][j] = w[j];
+    }
+  }
+}
+
+// The same for a matrix in memory that is too large to hold in registers beside the planes (N >
+// 4): two lines at a time, row by row.
+template <int N, bool FIRST, typename Real>
+__device__ __forceinline__ void lines_inplace_rows(const Real* p, Real (&X)[N][N]) {
+#pragma unroll
+  for (int l = 0; l < N; l += 2) {
+    constexpr int L = 2;
+    Real w[L][N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      Real row[N];
+      matrix_row<N>(p, j, row);
+#pragma unroll
+      for (int k = 0; k < L; ++k) {
+        if (l + k >= N) continue;
+        const int ll = l + k < N ? l + k : l;
+        Real s = row[0] * (FIRST ? X[0][ll] : X[ll][0]);
+#pragma unroll
+        for (int i = 1; i < N; ++i) s += row[i] * (FIRST ? X[i][ll] : X[ll][i]);
+        w[k][j] = s;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < L; ++k) {
+      if (l + k >= N) continue;
+      const int ll = l + k < N ? l + k : l;
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        if constexpr (FIRST) X[j][ll] = w[k][j];
+        else X[ll][j] = w[k][j];
+      }
+    }
+  }
+}
+
+// X <- A X along the first or second plane index, A in memory at p.
+template <int N, bool FIRST, typename Real>
+__device__ __forceinline__ void memory_pass(const Real* p, Real (&X)[N][N]) {
+  if constexpr (N <= 4) {
+    RegMat<N, Real> A;
+    load_matrix<N>(p, A);
+    lines_inplace<N, FIRST>(A, X);
+  } else {
+    lines_inplace_rows<N, FIRST>(p, X);
+  }
+}
+// Y <- A X along the second plane index, or Y += with ACC, A in memory at p.
+template <int N, bool ACC, typename Real>
+__device__ __forceinline__ void memory_pass_z(const Real* p, const Real (&X)[N][N], Real (&Y)[N][N]) {
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    Real row[N];
+    matrix_row<N>(p, k, row);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      Real s = ACC ? Y[i][k] : Real(0);
+#pragma unroll
+      for (int r = 0; r < N; ++r) s = (!ACC && r == 0) ? row[0] * X[i][0] : s + row[r] * X[i][r];
+      Y[i][k] = s;
+    }
+  }
+}
+
+// X <- (slot SLOT's matrix) X along the first or second plane index.
+template <int N, typename Real, int SLOT, bool FIRST, uint32_t VM>
+__device__ __forceinline__ void kron_pass(const KronParams<Real>& P, uint32_t coord, Real (&X)[N][N]) {
+  if (slot_varies<SLOT, VM>(P)) {
+    memory_pass<N, FIRST>(slot_matrix<SLOT>(P, coord), X);
+  } else {
+    lines_inplace<N, FIRST>(ParamMat<N, Real, SLOT>{P}, X);
+  }
+}
+
+// Y <- (slot SLOT's matrix) X along the second plane index, or Y += with ACC (the products
+// accumulate onto Y in one multiply-add chain per value).
+template <int N, typename Real, int SLOT, bool ACC, uint32_t VM>
+__device__ __forceinline__ void kron_pass_z(const KronParams<Real>& P, uint32_t coord, const Real (&X)[N][N],
+                                            Real (&Y)[N][N]) {
+  if (slot_varies<SLOT, VM>(P)) {
+    memory_pass_z<N, ACC>(slot_matrix<SLOT>(P, coord), X, Y);
+  } else {
+    const ParamMat<N, Real, SLOT> A{P};
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        Real s = ACC ? Y[i][k] : Real(0);
+#pragma unroll
+        for (int r = 0; r < N; ++r) s = (!ACC && r == 0) ? A(k, 0) * X[i][0] : s + A(k, r) * X[i][r];
+        Y[i][k] = s;
+      }
+  }
+}
+
+// One line: w = (slot SLOT's matrix) v.
+template <int N, typename Real, int SLOT, uint32_t VM>
+__device__ __forceinline__ void kron_line(const KronParams<Real>& P, uint32_t coord, const Real (&v)[N], Real (&w)[N]) {
+  if (slot_varies<SLOT, VM>(P)) {
+    const Real* p = slot_matrix<SLOT>(P, coord);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      Real row[N];
+      matrix_row<N>(p, j, row);
+      Real s = row[0] * v[0];
+#pragma unroll
+      for (int i = 1; i < N; ++i) s += row[i] * v[i];
+      w[j] = s;
+    }
+  } else {
+    const ParamMat<N, Real, SLOT> A{P};
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      Real s = A(j, 0) * v[0];
+#pragma unroll
+      for (int i = 1; i < N; ++i) s += A(j, i) * v[i];
+      w[j] = s;
+    }
+  }
+}
+
+template <int N, typename Real>
+__device__ __forceinline__ void copy_plane(const Real (&U)[N][N], Real (&X)[N][N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int j = 0; j < N; ++j) X[i][j] = U[i][j];
+}
+template <int N, typename Real>
+__device__ __forceinline__ void scale_plane(Real f, Real (&X)[N][N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int j = 0; j < N; ++j) X[i][j] *= f;
 }
 
 // Layout exchange between the N lanes of an element: X[i][j] held by lane t (plane index t of
@@ -324,33 +456,13 @@ __device__ __forceinline__ void load_plane_z(const Real* ub, int t, bool active,
     }
 }
 
-// Plane of an element in layout Y (values [x][z] of plane y = t) from the staged layout.
+// Layout exchange through the warp's shared tile: lane t holds X[i][j] = (x=i, y=j, z=t) and
+// receives X[i][k] = (x=i, y=t, z=k).  Tile layout [y][z][x].
 template <int N, typename Real>
-__device__ __forceinline__ void load_plane_y(const Real* ub, int t, bool active, Real (&u)[N][N]) {
-  using S = Kron3DShape<N, Real>;
-  constexpr int V = S::V;
-#pragma unroll
-  for (int k = 0; k < N; ++k)
-#pragma unroll
-    for (int i = 0; i < N; i += V) {
-      Real v[V];
-      if (active) vload<Real, V>(ub + k * S::SP + N * t + i, v);
-#pragma unroll
-      for (int q = 0; q < V; ++q) u[i + q][k] = active ? v[q] : Real(0);
-    }
-}
-
-// Layout exchange through the warp's shared tile.  z_to_y: lane t holds X[i][j] = (x=i, y=j, z=t)
-// and receives X[i][k] = (x=i, y=t, z=k); otherwise the reverse.  Tile layout [y][z][x].
-template <int N, typename Real>
-__device__ __forceinline__ void exchange_tile(Real* tile, int le, int t, bool slot, bool z_to_y, Real (&X)[N][N]) {
+__device__ __forceinline__ void exchange_tile(Real* tile, int le, int t, bool slot, Real (&X)[N][N]) {
   using S = Kron3DShape<N, Real>;
   constexpr int V = S::V;
   Real* b = tile + le * S::TSE;
-  // layout Z side: lane t = z owns (x, y = j) at j * TA + t * N + x;
-  // layout Y side: lane t = y owns (x, z = k) at t * TA + k * N + x
-  auto z_side = [&](int j, int i) { return b + j * S::TA + t * N + i; };
-  auto y_side = [&](int k, int i) { return b + t * S::TA + k * N + i; };
   if (slot) {
 #pragma unroll
     for (int j = 0; j < N; ++j)
@@ -359,19 +471,19 @@ __device__ __forceinline__ void exchange_tile(Real* tile, int le, int t, bool sl
         Real v[V];
 #pragma unroll
         for (int q = 0; q < V; ++q) v[q] = X[i + q][j];
-        vstore<Real, V>(z_to_y ? z_side(j, i) : y_side(j, i), v);
+        vstore<Real, V>(b + j * S::TA + t * N + i, v);
       }
   }
   __syncwarp();
   if (slot) {
 #pragma unroll
-    for (int j = 0; j < N; ++j)
+    for (int k = 0; k < N; ++k)
 #pragma unroll
       for (int i = 0; i < N; i += V) {
         Real v[V];
-        vload<Real, V>(z_to_y ? y_side(j, i) : z_side(j, i), v);
+        vload<Real, V>(b + t * S::TA + k * N + i, v);
 #pragma unroll
-        for (int q = 0; q < V; ++q) X[i + q][j] = v[q];
+        for (int q = 0; q < V; ++q) X[i + q][k] = v[q];
       }
   }
   __syncwarp();  // the tile is free again
@@ -443,23 +555,63 @@ __device__ __forceinline__ Real tan_sign(const KronParams<Real>& P, int a, const
   return s;
 }
 
-// Is the x neighbour on side s the adjacent element of the same staged group?
-__device__ __forceinline__ bool x_in_group(int s, int le, int ne, uint32_t cx, int64_t nx) {
-  const int rl = le + (s ? 1 : -1);
-  return rl >= 0 && rl < ne && (s ? (int64_t)cx + 1 < nx : cx > 0);
-}
-
-enum TraceSrc { kTraceLocal = 0, kTraceSlot = 1, kTraceGlobal = 2 };
-// Face record bits (5 per face f = axis * 2 + side): corner, neighbour trace, inflow value g,
-// and the trace source (TraceSrc) in bits 3-4.
-enum : uint32_t { kRecCorner = 1u, kRecNb = 2u, kRecG = 4u };
+// Face word of an element: 3 bits per face f = 2 axis + side (own trace of an outflow face, the
+// neighbour's trace, the inflow value), and bit kFaceWrap + f when that face's neighbour lies
+// across a periodic boundary.
+enum : uint32_t { kFaceCorner = 1u, kFaceNb = 2u, kFaceG = 4u };
+constexpr int kFaceWrap = 18;
 
 template <typename Real>
-__device__ __forceinline__ int64_t neighbour_offset(const KronParams<Real>& P, int a, int s, uint32_t ca) {
-  const int64_t n = P.sizes[a];
+__device__ __forceinline__ uint32_t face_word(const KronParams<Real>& P, int64_t e, const uint32_t (&c)[3]) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const Real tsign = tan_sign(P, a, c);
+    const Real el = P.elem[a] ? P.elem[a][e] : Real(1);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      Real phi, coef;
+      const FaceDecision f = face_decide(P, a, s, c, e, tsign, el, phi, coef);
+      const uint32_t b = (f.corner ? kFaceCorner : 0u) | (f.use_nb ? kFaceNb : 0u) | (f.use_g ? kFaceG : 0u);
+      const bool wrap = s == 0 ? c[a] == 0 : (int64_t)c[a] + 1 == P.sizes[a];
+      w |= b << (3 * (2 * a + s)) | (wrap ? 1u << (kFaceWrap + 2 * a + s) : 0u);
+    }
+  }
+  return w;
+}
+// With per-element velocity factors, whose values (and signs) the caller may change between
+// applies: the word from the factors' current values.
+template <typename Real>
+__device__ __noinline__ uint32_t face_word_now(const KronParams<Real>& P, int64_t e) {
+  uint32_t c[3];
+  kron_coords(P, (uint32_t)e, c);
+  return face_word(P, e, c);
+}
+template <typename Real>
+__device__ __forceinline__ uint32_t load_face_word(const KronParams<Real>& P, int64_t e) {
+  return P.eflags ? __ldg(P.eflags + e) : face_word_now(P, e);
+}
+__device__ __forceinline__ uint32_t face_bits(uint32_t w, int a, int s) { return (w >> (3 * (2 * a + s))) & 7u; }
+__device__ __forceinline__ bool face_wraps(uint32_t w, int a, int s) {
+  return ((w >> (kFaceWrap + 2 * a + s)) & 1u) != 0;
+}
+
+// Element offset to the neighbour across face (a, s).
+template <typename Real>
+__device__ __forceinline__ int64_t face_offset(const KronParams<Real>& P, uint32_t w, int a, int s) {
   const int64_t st = a == 0 ? 1 : (a == 1 ? P.sizes[0] : P.sizes[0] * P.sizes[1]);
-  if (s == 0) return ca > 0 ? -st : (n - 1) * st;
-  return (int64_t)ca + 1 < n ? st : -(n - 1) * st;
+  const int64_t d = face_wraps(w, a, s) ? -(P.sizes[a] - 1) * st : st;
+  return s ? d : -d;
+}
+// Coefficient of the neighbour's trace on face (a, s): the element's own phi (forward) or, transposed,
+// the neighbour's at its opposite face, times the per-element factor.
+template <typename Real>
+__device__ __forceinline__ Real face_nb_coef(const KronParams<Real>& P, uint32_t w, int a, int s, uint32_t ca, int64_t e,
+                                             Real k_own) {
+  if (!(P.flags & kTranspose)) return k_own;
+  const uint32_t cn = face_wraps(w, a, s) ? (s ? 0u : (uint32_t)(P.sizes[a] - 1)) : (s ? ca + 1 : ca - 1);
+  const Real phin = P.phi[a][cn * 2 + (1 - s)];
+  return P.elem[a] ? phin * P.elem[a][e + face_offset(P, w, a, s)] : phin;
 }
 
 // One staged neighbour-trace row (N Reals), V-wide.
@@ -475,45 +627,125 @@ __device__ __forceinline__ void trace_row(const Real* p, Real (&v)[N]) {
   }
 }
 
-// Face terms of axis a added to a D-pass output Pm (plane [first][second]; the face slice is along
-// the first index when FIRST), from the element's face record (see stage_group).  nbrow(side, src,
-// e_nb, v) reads this lane's row of the neighbour trace of that side from the group's staged DoFs
-// (x only), the axis' staged trace slot (V-wide), or global memory.
-template <int N, typename Real, bool FIRST, typename NbRow>
-__device__ __forceinline__ void kron_faces(const KronParams<Real>& P, int a, const uint32_t (&c)[3], int64_t e,
-                                           uint32_t flags, const Real* rec, const Real (&U)[N][N], Real (&Pm)[N][N],
-                                           NbRow nbrow) {
+// Face terms of axis a (0 or 1) added to the D-pass output X of plane z = t (the face slice is along
+// the first index for a = 0, the second for a = 1).  own(i, j): the input plane's values;
+// nbrow(s, v): this lane's row of the neighbour's trace on its opposite face.  The trace is the
+// slice there, or with GL (a basis without nodes on the faces) the plane's lines times the basis
+// values P.lf, and a face term goes to every slice with those weights.
+template <int N, typename Real, int A, bool GL, typename Own, typename NbRow>
+__device__ __forceinline__ void plane_faces(const KronParams<Real>& P, uint32_t ca, int64_t e, uint32_t w,
+                                            Real (&X)[N][N], Own own, NbRow nbrow) {
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
+    const uint32_t f = face_bits(w, A, s);
+    if (!f) continue;
     const int sl = s ? N - 1 : 0;
-    const uint32_t f = (flags >> (5 * (a * 2 + s))) & 31u;
-    if (f & kRecCorner) {
-      const Real k = rec[(a * 2 + s) * 2];
+    Real k = P.phi[A][ca * 2 + s];
+    if (P.elem[A]) k *= P.elem[A][e];
+    auto add = [&](Real kk, const Real(&v)[N]) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if (!GL && i != sl) continue;
+        const Real ki = GL ? kk * P.lf[s][i] : kk;
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+          if constexpr (A == 0) X[i][r] += ki * v[r];
+          else X[r][i] += ki * v[r];
+        }
+      }
+    };
+    if (f & kFaceCorner) {
+      Real v[N];
 #pragma unroll
       for (int r = 0; r < N; ++r) {
-        if (FIRST) Pm[sl][r] += k * U[sl][r];
-        else Pm[r][sl] += k * U[r][sl];
-      }
-    }
-    if (f & (kRecNb | kRecG)) {
-      const Real k = rec[(a * 2 + s) * 2 + 1];
-      if (f & kRecNb) {
-        const int src = (int)(f >> 3);
-        const int64_t en = src == kTraceGlobal ? e + neighbour_offset(P, a, s, c[a]) : e;
-        Real v[N];
-        nbrow(s, src, en, v);
+        if constexpr (GL) {
+          v[r] = Real(0);
 #pragma unroll
-        for (int r = 0; r < N; ++r) {
-          if (FIRST) Pm[sl][r] += k * v[r];
-          else Pm[r][sl] += k * v[r];
+          for (int i = 0; i < N; ++i) v[r] += P.lf[s][i] * (A == 0 ? own(i, r) : own(r, i));
+        } else {
+          v[r] = A == 0 ? own(sl, r) : own(r, sl);
         }
+      }
+      add(k, v);
+    }
+    if (f & (kFaceNb | kFaceG)) {
+      Real v[N];
+      if (f & kFaceNb) {
+        k = face_nb_coef(P, w, A, s, ca, e, k);
+        nbrow(s, v);
       } else {
 #pragma unroll
-        for (int r = 0; r < N; ++r) {
-          if (FIRST) Pm[sl][r] += k * P.g;
-          else Pm[r][sl] += k * P.g;
+        for (int r = 0; r < N; ++r) v[r] = P.g;
+      }
+      add(k, v);
+    }
+  }
+}
+
+// The z faces' neighbour traces through Tzy: col(s, v) reads column x = t (values y) of the z
+// neighbour's opposite slice, put(s, w) stores the result column in place of it.
+template <int N, typename Real, uint32_t VM, typename Col, typename Put>
+__device__ __forceinline__ void z_faces_prepare(const KronParams<Real>& P, const uint32_t (&c)[3], int64_t e,
+                                                uint32_t w, Col col, Put put) {
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const uint32_t f = face_bits(w, 2, s);
+    if (!(f & (kFaceNb | kFaceG))) continue;
+    Real k = P.phi[2][c[2] * 2 + s];
+    if (P.elem[2]) k *= P.elem[2][e];
+    Real v[N], r[N];
+    if (f & kFaceNb) {
+      k = face_nb_coef(P, w, 2, s, c[2], e, k);
+      col(s, v);
+    } else {
+#pragma unroll
+      for (int y = 0; y < N; ++y) v[y] = P.g;
+    }
+    kron_line<N, Real, kSlotTZY, VM>(P, c[1], v, r);
+#pragma unroll
+    for (int y = 0; y < N; ++y) r[y] *= k;
+    put(s, r);
+  }
+}
+// Z-face terms added to the accumulator in layout Y: the own trace of an outflow face (X: the z
+// term's lines before Dz, already scaled by the element's factor) and row y = t of the prepared
+// neighbour traces (row(s, v)) through Tzx.
+template <int N, typename Real, uint32_t VM, bool GL, typename Row>
+__device__ __forceinline__ void z_faces_add(const KronParams<Real>& P, const uint32_t (&c)[3], uint32_t w,
+                                            const Real (&X)[N][N], Real (&out)[N][N], Row row) {
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const uint32_t f = face_bits(w, 2, s);
+    if (!f) continue;
+    const int sl = s ? N - 1 : 0;
+    auto add = [&](int i, Real v) {
+      if constexpr (GL) {
+#pragma unroll
+        for (int z = 0; z < N; ++z) out[i][z] += P.lf[s][z] * v;
+      } else {
+        out[i][sl] += v;
+      }
+    };
+    if (f & kFaceCorner) {
+      const Real k = P.phi[2][c[2] * 2 + s];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        if constexpr (GL) {
+          Real tr = Real(0);
+#pragma unroll
+          for (int z = 0; z < N; ++z) tr += P.lf[s][z] * X[i][z];
+          add(i, k * tr);
+        } else {
+          out[i][sl] += k * X[i][sl];
         }
       }
+    }
+    if (f & (kFaceNb | kFaceG)) {
+      Real v[N], r[N];
+      row(s, v);
+      kron_line<N, Real, kSlotTZX, VM>(P, c[0], v, r);
+#pragma unroll
+      for (int i = 0; i < N; ++i) add(i, r[i]);
     }
   }
 }
@@ -542,56 +774,42 @@ __device__ __forceinline__ void copy_row(Real* dst, const Real* src) {
   for (int i = 0; i < N; i += R) cp_async<S::RB>(dst + i, src + i);
 }
 
-// Stage the DoFs of elements [e0, e0 + ne) into `buf` (padded layout, coalesced); for advection,
-// also each element's face record and the neighbour traces its faces will read (lane t copies
-// row t of each trace).
+// Where x face s of an element finds its neighbour's trace: the adjacent element of the same
+// staged group, trace slot 0 (the first face that is not in the group), or global memory.
+__device__ __forceinline__ bool x_in_group(uint32_t w, int s, int le, int ne) {
+  return !face_wraps(w, 0, s) && (s ? le + 1 < ne : le > 0);
+}
+__device__ __forceinline__ bool x_slot_taken(uint32_t w, int le, int ne) {  // by face 0
+  return (face_bits(w, 0, 0) & kFaceNb) && !x_in_group(w, 0, le, ne);
+}
+
+// Stage the DoFs of elements [e0, e0 + ne) into `buf` (padded layout, coalesced) and, for
+// advection, the neighbour traces the faces in word w will read (lane t copies row t of each).
 template <int N, typename Real>
 __device__ __forceinline__ void stage_group(const KronParams<Real>& P, int64_t e0, int ne, Real* buf, int lane,
-                                            int le, int t, bool adv) {
+                                            int le, int t, uint32_t w, bool traces = true) {
   using S = Kron3DShape<N, Real>;
   const int nchunks = ne * S::NNN / S::CR;
   const Real* src = P.x + e0 * S::NNN;
   for (int ch = lane; ch < nchunks; ch += 32) {
     const int d = ch * S::CR;
     const int r = d / S::NNN, o = d - r * S::NNN;
-    const int z = o / S::NN, w = o - z * S::NN;
-    cp_async<S::CB>(buf + r * S::SE + z * S::SP + w, src + d);
+    const int z = o / S::NN, q = o - z * S::NN;
+    cp_async<S::CB>(buf + r * S::SE + z * S::SP + q, src + d);
   }
-  if (!adv || le >= ne) return;
-  const int64_t e = e0 + le;
-  uint32_t c[3];
-  kron_coords(P, (uint32_t)e, c);
+  if (!w || le >= ne || !traces) return;
+  const Real* ue = P.x + (e0 + le) * S::NNN;
   Real* tb = buf + S::EPW * S::SE + le * S::TE;
-  Real* rb = buf + S::EPW * (S::SE + S::TE) + le * S::RE;
-  uint32_t flags = 0;
 #pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    const Real tsign = tan_sign(P, a, c);
-    const Real el = P.elem[a] ? P.elem[a][e] : Real(1);
-    bool slot_taken = false;
+  for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
-      Real phi, coef;
-      const FaceDecision f = face_decide(P, a, s, c, e, tsign, el, phi, coef);
-      uint32_t bits = 0;
-      if (f.corner) bits |= kRecCorner;
-      if (f.use_g) bits |= kRecG;
-      int src = kTraceLocal;
-      if (f.use_nb) {
-        bits |= kRecNb;
-        if (!(a == 0 && x_in_group(s, le, ne, c[0], P.sizes[0]))) src = slot_taken ? kTraceGlobal : kTraceSlot;
-      }
-      bits |= (uint32_t)src << 3;
-      flags |= bits << (5 * (a * 2 + s));
-      if (t == 0) {
-        rb[(a * 2 + s) * 2] = phi * el;
-        rb[(a * 2 + s) * 2 + 1] = coef;
-      }
-      if (src != kTraceSlot) continue;  // staged DoFs (x neighbours in the group) or global memory
-      slot_taken = true;
-      const Real* un = P.x + (e + f.d) * S::NNN;
+      if (!(face_bits(w, a, s) & kFaceNb)) continue;
+      if (a == 0 && (x_in_group(w, s, le, ne) || (s == 1 && x_slot_taken(w, le, ne)))) continue;
+      if (a == 1 && s == 1 && (face_bits(w, 1, 0) & kFaceNb)) continue;
+      const Real* un = ue + face_offset(P, w, a, s) * S::NNN;
       const int sl = s ? 0 : N - 1;  // the neighbour's opposite slice
-      Real* dst = tb + a * S::TS + t * S::TR;
+      Real* dst = tb + (a == 2 ? 2 + s : a) * S::TS + t * S::TR;
       if (a == 0) {
 #pragma unroll
         for (int r = 0; r < N; ++r) cp_async<(int)sizeof(Real)>(dst + r, un + sl + N * r + S::NN * t);
@@ -601,8 +819,6 @@ __device__ __forceinline__ void stage_group(const KronParams<Real>& P, int64_t e
         copy_row<N>(dst, un + N * t + S::NN * sl);
       }
     }
-  }
-  if (t == 0) *reinterpret_cast<uint32_t*>(rb + 12) = flags;
 }
 
 constexpr int kron_max_warps = 4;  // warps per CTA of kron3d_kernel (128 threads)
@@ -613,7 +829,9 @@ constexpr int kron_max_warps = 4;  // warps per CTA of kron3d_kernel (128 thread
 //   SHFL:    layout exchanges by shuffle butterflies (even N) instead of the shared tile
 //   DOT:     the inner-product epilogue (P.dot_partials; FP64 solvers) is compiled in
 //   VM:      the slot mask the kernel is compiled for (kVaryRuntime: read P.vary)
-template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT, uint32_t VM>
+//   GEN:     the general form: with P.gl a basis without nodes on the faces (the neighbours' traces
+//            are formed from their whole elements, read from global memory), and P.nextra mass terms
+template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT, uint32_t VM, bool GEN>
 __device__ __forceinline__ void kron3d_body(const KronParams<Real>& P) {
   using S = Kron3DShape<N, Real>;
   constexpr int NN = S::NN, NNN = S::NNN, EPW = S::EPW;
@@ -627,203 +845,217 @@ __device__ __forceinline__ void kron3d_body(const KronParams<Real>& P) {
   const int64_t nwarps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const bool adv = P.has_adv != 0;
   const bool slot = le < EPW;
+  const bool gl = GEN && P.gl;
   if (P.skip && *P.skip) return;  // a finished solve: nothing to do
   [[maybe_unused]] double dot_acc = 0.0;
 
+  auto first_of = [&](int64_t g) { return P.e_begin + g * EPW; };
+  // this lane's face word in group g (0: no element, or no faces)
+  auto word_of = [&](int64_t g) -> uint32_t {
+    const int64_t e = first_of(g) + le;
+    return (adv && slot && g < ngroups && e < P.nelem) ? load_face_word(P, e) : 0u;
+  };
+  auto exchange = [&](Real(&X)[N][N]) {
+    if constexpr (BFLY) exchange_butterfly<N>(t, X);
+    else exchange_tile<N>(tile, le, t, slot, X);
+  };
+
   int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
+  // face words: of this group and of the next one to be staged, loaded ahead of its copies
+  uint32_t w = word_of(g), w_next = STAGES == 2 ? word_of(g + nwarps) : 0u;
   if constexpr (STAGES == 2) {
-    if (g < ngroups) stage_group<N>(P, P.e_begin + g * EPW, group_size(EPW, P.nelem - P.e_begin - g * EPW), wbase, lane, le, t, adv);
+    if (g < ngroups) stage_group<N>(P, first_of(g), group_size(EPW, P.nelem - first_of(g)), wbase, lane, le, t, w, !gl);
     cp_async_commit();
   }
   for (int it = 0; g < ngroups; g += nwarps, ++it) {
     Real* buf = wbase + (STAGES == 2 ? (it & 1) * S::STAGE : 0);
+    const uint32_t wc = w;
     if constexpr (STAGES == 2) {
       const int64_t gn = g + nwarps;
       if (gn < ngroups)
-        stage_group<N>(P, P.e_begin + gn * EPW, group_size(EPW, P.nelem - P.e_begin - gn * EPW), wbase + ((it + 1) & 1) * S::STAGE, lane, le,
-                       t, adv);
+        stage_group<N>(P, first_of(gn), group_size(EPW, P.nelem - first_of(gn)), wbase + ((it + 1) & 1) * S::STAGE, lane,
+                       le, t, w_next, !gl);
       cp_async_commit();
+      w = w_next;
+      w_next = word_of(gn + nwarps);
       cp_async_wait<1>();
     } else {
-      stage_group<N>(P, P.e_begin + g * EPW, group_size(EPW, P.nelem - P.e_begin - g * EPW), buf, lane, le, t, adv);
+      stage_group<N>(P, first_of(g), group_size(EPW, P.nelem - first_of(g)), buf, lane, le, t, wc, !gl);
       cp_async_commit();
+      w = word_of(g + nwarps);
       cp_async_wait<0>();
     }
     __syncwarp();
-    const int64_t e0 = P.e_begin + g * EPW;
+    const int64_t e0 = first_of(g);
     const int ne = group_size(EPW, P.nelem - e0);
     const int64_t e = e0 + le;
     const bool active = slot && le < ne;
     uint32_t c[3] = {0, 0, 0};
     if (active) kron_coords(P, (uint32_t)e, c);
     const Real* ub = buf + (slot ? le : 0) * S::SE;
-    const Real* tb = buf + EPW * S::SE + (slot ? le : 0) * S::TE;
-    const Real* rec = buf + EPW * (S::SE + S::TE) + (slot ? le : 0) * S::RE;
-    const uint32_t fflags = (adv && active) ? *reinterpret_cast<const uint32_t*>(rec + 12) : 0u;
-    Real qx[N][N], py[N][N];
+    Real* tb = buf + EPW * S::SE + (slot ? le : 0) * S::TE;
+    // the input plane: held in registers (one shared-memory read for all terms) in the forms whose
+    // registers allow it, otherwise read again by each term
+    constexpr bool KEEP = N <= 4 && VM != kVaryRuntime && !SEP;
+    [[maybe_unused]] Real U[KEEP ? N : 1][KEEP ? N : 1];
+    if constexpr (KEEP) load_plane_z<N>(ub, t, active, U);
+    auto input = [&](Real(&X)[N][N]) {
+      if constexpr (KEEP) copy_plane<N>(U, X);
+      else load_plane_z<N>(ub, t, active, X);
+    };
+    auto own = [&](int i, int j) {
+      if constexpr (KEEP) return U[i][j];
+      else return ub[t * S::SP + N * j + i];
+    };
+    Real out[N][N];
 
-    // ------------------------------------------------------------ layout Z (plane z = t)
     if (adv) {
-      Real u[N][N];
-      load_plane_z<N>(ub, t, active, u);
+      if (wc)
+        z_faces_prepare<N, Real, VM>(
+            P, c, e, wc,
+            [&](int s, Real(&v)[N]) {
+              if (GEN && gl) {
+                const Real* un = P.x + (e + face_offset(P, wc, 2, s)) * NNN + t;
+#pragma unroll
+                for (int y = 0; y < N; ++y) v[y] = Real(0);
+#pragma unroll
+                for (int z = 0; z < N; ++z)
+#pragma unroll
+                  for (int y = 0; y < N; ++y) v[y] += P.lf[1 - s][z] * un[N * y + NN * z];
+                return;
+              }
+#pragma unroll
+              for (int y = 0; y < N; ++y) v[y] = tb[(2 + s) * S::TS + y * S::TR + t];
+            },
+            [&](int s, const Real(&r)[N]) {
+#pragma unroll
+              for (int y = 0; y < N; ++y) tb[(2 + s) * S::TS + y * S::TR + t] = r[y];
+            });
+      // ---------------------------------------------------------------- x term
       {
-        Real px[N][N];
-        kron_apply<N, Real, kSlotDX, true, VM>(P, c[0], u, px);
-        if (P.elem[0]) {
-          const Real elx = active ? P.elem[0][e] : Real(1);
+        Real X[N][N];
+        input(X);
+        if (P.elem[0]) scale_plane<N>(active ? P.elem[0][e] : Real(1), X);
+        kron_pass<N, Real, kSlotDX, true, VM>(P, c[0], X);
+        if (GEN && gl) {
+          if (wc)
+            plane_faces<N, Real, 0, true>(P, c[0], e, wc, X, own, [&](int s, Real(&v)[N]) {
+              const Real* un = P.x + (e + face_offset(P, wc, 0, s)) * NNN + NN * t;
 #pragma unroll
-          for (int i = 0; i < N; ++i)
+              for (int r = 0; r < N; ++r) {
+                v[r] = Real(0);
 #pragma unroll
-            for (int j = 0; j < N; ++j) px[i][j] *= elx;
-        }
-        if (active)
-          kron_faces<N, Real, true>(P, 0, c, e, fflags, rec, u, px, [&](int s, int src, int64_t en, Real(&v)[N]) {
+                for (int i = 0; i < N; ++i) v[r] += P.lf[1 - s][i] * un[i + N * r];
+              }
+            });
+        } else if (wc) {
+          plane_faces<N, Real, 0, false>(P, c[0], e, wc, X, own, [&](int s, Real(&v)[N]) {
             const int sl = s ? 0 : N - 1;  // the neighbour's opposite slice
-            if (src == kTraceSlot) {
-              trace_row<N>(tb + 0 * S::TS + t * S::TR, v);
-            } else {
+            if (x_in_group(wc, s, le, ne)) {
 #pragma unroll
-              for (int r = 0; r < N; ++r)
-                v[r] = src == kTraceLocal ? ub[(s ? 1 : -1) * S::SE + t * S::SP + sl + N * r]
-                                          : P.x[en * NNN + sl + N * r + NN * t];
+              for (int r = 0; r < N; ++r) v[r] = ub[(s ? S::SE : -S::SE) + t * S::SP + sl + N * r];
+            } else if (s == 0 || !x_slot_taken(wc, le, ne)) {
+              trace_row<N>(tb + t * S::TR, v);
+            } else {
+              const Real* un = P.x + (e + face_offset(P, wc, 0, s)) * NNN;
+#pragma unroll
+              for (int r = 0; r < N; ++r) v[r] = un[sl + N * r + NN * t];
             }
           });
-        kron_apply<N, Real, kSlotTXY, false, VM>(P, c[1], px, qx);
-      }
-      kron_apply<N, Real, kSlotDY, false, VM>(P, c[1], u, py);
-      if (P.elem[1]) {
-        const Real ely = active ? P.elem[1][e] : Real(1);
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-          for (int j = 0; j < N; ++j) py[i][j] *= ely;
-      }
-      if (active)
-        kron_faces<N, Real, false>(P, 1, c, e, fflags, rec, u, py, [&](int s, int src, int64_t en, Real(&v)[N]) {
-          if (src == kTraceSlot) {
-            trace_row<N>(tb + 1 * S::TS + t * S::TR, v);
-          } else {
-#pragma unroll
-            for (int r = 0; r < N; ++r) v[r] = P.x[en * NNN + r + N * (s ? 0 : N - 1) + NN * t];
-          }
-        });
-      if constexpr (BFLY) {
-        exchange_butterfly<N>(t, qx);
-        exchange_butterfly<N>(t, py);
-      } else {
-        exchange_tile<N>(tile, le, t, slot, true, qx);
-        exchange_tile<N>(tile, le, t, slot, true, py);
-      }
-    }
-
-    // ------------------------------------------------------------ layout Y (plane y = t)
-    Real out[N][N], qz[N][N];
-    [[maybe_unused]] Real qm[N][N];
-    {
-      // x and y terms first, so their inputs die before u is loaded
-      if (adv) {
-        kron_apply<N, Real, kSlotTXZ, false, VM>(P, c[2], qx, out);
-        kron_apply<N, Real, kSlotTYZ, false, VM>(P, c[2], py, qx);  // qx reused as scratch
-        kron_apply<N, Real, kSlotTYX, true, VM>(P, c[0], qx, py);
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-          for (int k = 0; k < N; ++k) out[i][k] += py[i][k];
-      } else {
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-          for (int k = 0; k < N; ++k) out[i][k] = Real(0);
-      }
-      Real u[N][N], pz[N][N];
-      load_plane_y<N>(ub, t, active, u);
-      kron_apply<N, Real, kSlotDZ, false, VM>(P, c[2], u, pz);
-      if (adv) {
-        if (P.elem[2]) {
-          const Real elz = active ? P.elem[2][e] : Real(1);
-#pragma unroll
-          for (int i = 0; i < N; ++i)
-#pragma unroll
-            for (int k = 0; k < N; ++k) pz[i][k] *= elz;
         }
-        if (active)
-          kron_faces<N, Real, false>(P, 2, c, e, fflags, rec, u, pz, [&](int s, int src, int64_t en, Real(&v)[N]) {
-            if (src == kTraceSlot) {
-              trace_row<N>(tb + 2 * S::TS + t * S::TR, v);
-            } else {
+        kron_pass<N, Real, kSlotTXY, false, VM>(P, c[1], X);
+        exchange(X);
+        kron_pass_z<N, Real, kSlotTXZ, false, VM>(P, c[2], X, out);
+      }
+      // ---------------------------------------------------------------- y term
+      {
+        Real X[N][N];
+        input(X);
+        if (P.elem[1]) scale_plane<N>(active ? P.elem[1][e] : Real(1), X);
+        kron_pass<N, Real, kSlotDY, false, VM>(P, c[1], X);
+        if (GEN && gl) {
+          if (wc)
+            plane_faces<N, Real, 1, true>(P, c[1], e, wc, X, own, [&](int s, Real(&v)[N]) {
+              const Real* un = P.x + (e + face_offset(P, wc, 1, s)) * NNN + NN * t;
 #pragma unroll
-              for (int r = 0; r < N; ++r) v[r] = P.x[en * NNN + r + N * t + NN * (s ? 0 : N - 1)];
+              for (int r = 0; r < N; ++r) v[r] = Real(0);
+#pragma unroll
+              for (int y = 0; y < N; ++y)
+#pragma unroll
+                for (int r = 0; r < N; ++r) v[r] += P.lf[1 - s][y] * un[r + N * y];
+            });
+        } else if (wc) {
+          plane_faces<N, Real, 1, false>(P, c[1], e, wc, X, own, [&](int s, Real(&v)[N]) {
+            if (s == 0 || !(face_bits(wc, 1, 0) & kFaceNb)) {
+              trace_row<N>(tb + S::TS + t * S::TR, v);
+            } else {
+              const Real* un = P.x + (e + face_offset(P, wc, 1, s)) * NNN;
+#pragma unroll
+              for (int r = 0; r < N; ++r) v[r] = un[r + N * (s ? 0 : N - 1) + NN * t];
             }
           });
-      } else if (P.elem_mass) {
-        const Real em = active ? P.elem_mass[e] : Real(1);
-#pragma unroll
-        for (int i = 0; i < N; ++i)
-#pragma unroll
-          for (int k = 0; k < N; ++k) pz[i][k] *= em;
-      }
-      kron_apply<N, Real, kSlotTZX, true, VM>(P, c[0], pz, qz);
-      if constexpr (SEP) {
-        kron_apply<N, Real, kSlotMD, false, VM>(P, c[2], u, pz);
-        if (P.elem_mass) {
-          const Real em = active ? P.elem_mass[e] : Real(1);
-#pragma unroll
-          for (int i = 0; i < N; ++i)
-#pragma unroll
-            for (int k = 0; k < N; ++k) pz[i][k] *= em;
         }
-        kron_apply<N, Real, kSlotMX, true, VM>(P, c[0], pz, qm);
+        kron_pass<N, Real, kSlotTYX, true, VM>(P, c[0], X);
+        exchange(X);
+        kron_pass_z<N, Real, kSlotTYZ, true, VM>(P, c[2], X, out);
       }
-    }
-    __syncwarp();  // every lane is done reading the staged input of this group
-    Real* ob = buf + le * S::SE;  // output staging: the group's DoF slots, staged layout
-    if constexpr (BFLY) {
-      exchange_butterfly<N>(t, qz);
-      exchange_butterfly<N>(t, out);
-      if constexpr (SEP) exchange_butterfly<N>(t, qm);
     } else {
-      // x and y terms leave in layout Y straight to the output slots; the z term crosses to
-      // layout Z through the tile and is added there
-      if (slot) {
-#pragma unroll
-        for (int k = 0; k < N; ++k)
-#pragma unroll
-          for (int i = 0; i < N; i += S::V) {
-            Real v[S::V];
-#pragma unroll
-            for (int q = 0; q < S::V; ++q) v[q] = out[i + q][k];
-            vstore<Real, S::V>(ob + k * S::SP + N * t + i, v);
-          }
-      }
-      exchange_tile<N>(tile, le, t, slot, false, qz);
-      if constexpr (SEP) exchange_tile<N>(tile, le, t, slot, false, qm);
-    }
-
-    // ------------------------------------------------------------ layout Z, output
-    kron_apply<N, Real, kSlotTZY, false, VM>(P, c[1], qz, py);
-    if constexpr (SEP) {
-      kron_apply<N, Real, kSlotMY, false, VM>(P, c[1], qm, qx);
 #pragma unroll
       for (int i = 0; i < N; ++i)
 #pragma unroll
-        for (int j = 0; j < N; ++j) py[i][j] += qx[i][j];
+        for (int k = 0; k < N; ++k) out[i][k] = Real(0);
     }
-    if (slot) {
-      Real* op = ob + t * S::SP;
+    // ------------------------------------------------ z term (with a merged mass), or the mass term
+    if (!GEN || adv || P.nextra == 0) {
+      Real X[N][N];
+      input(X);
+      const Real* ez = adv ? P.elem[2] : P.elem_mass;
+      if (ez) scale_plane<N>(active ? ez[e] : Real(1), X);
+      kron_pass<N, Real, kSlotTZX, true, VM>(P, c[0], X);
+      kron_pass<N, Real, kSlotTZY, false, VM>(P, c[1], X);
+      exchange(X);
+      kron_pass_z<N, Real, kSlotDZ, true, VM>(P, c[2], X, out);
+      if constexpr (BFLY) __syncwarp();  // the z traces' other columns (the tile exchange synchronizes)
+      auto z_row = [&](int s, Real(&v)[N]) { trace_row<N>(tb + (2 + s) * S::TS + t * S::TR, v); };
+      if (GEN && gl) {
+        if (wc) z_faces_add<N, Real, VM, true>(P, c, wc, X, out, z_row);
+      } else if (wc) {
+        z_faces_add<N, Real, VM, false>(P, c, wc, X, out, z_row);
+      }
+    }
+    if constexpr (GEN) {
+      // the mass terms of a density that is a sum of products
+      for (int m = 0; m < P.nextra; ++m) {
+        auto matrix = [&](int k) { return P.mats + P.extra[m][k].off + (int64_t)c[k] * P.extra[m][k].stride; };
+        Real X[N][N];
+        input(X);
+        if (P.elem_mass) scale_plane<N>(active ? P.elem_mass[e] : Real(1), X);
+        memory_pass<N, true>(matrix(0), X);
+        memory_pass<N, false>(matrix(1), X);
+        exchange(X);
+        memory_pass_z<N, true>(matrix(2), X, out);
+      }
+    }
+    if constexpr (SEP) {
+      Real X[N][N];
+      input(X);
+      if (P.elem_mass) scale_plane<N>(active ? P.elem_mass[e] : Real(1), X);
+      kron_pass<N, Real, kSlotMX, true, VM>(P, c[0], X);
+      kron_pass<N, Real, kSlotMY, false, VM>(P, c[1], X);
+      exchange(X);
+      kron_pass_z<N, Real, kSlotMD, true, VM>(P, c[2], X, out);
+    }
+    __syncwarp();  // every lane is done reading the staged input of this group
+    if (slot) {    // output staging: the group's DoF slots, staged layout
+      Real* ob = buf + le * S::SE;
 #pragma unroll
-      for (int j = 0; j < N; ++j)
+      for (int k = 0; k < N; ++k)
 #pragma unroll
         for (int i = 0; i < N; i += S::V) {
           Real v[S::V];
-          if constexpr (BFLY) {
 #pragma unroll
-            for (int q = 0; q < S::V; ++q) v[q] = out[i + q][j] + py[i + q][j];
-          } else {
-            vload<Real, S::V>(op + N * j + i, v);
-#pragma unroll
-            for (int q = 0; q < S::V; ++q) v[q] += py[i + q][j];
-          }
-          vstore<Real, S::V>(op + N * j + i, v);
+          for (int q = 0; q < S::V; ++q) v[q] = out[i + q][k];
+          vstore<Real, S::V>(ob + k * S::SP + N * t + i, v);
         }
     }
     __syncwarp();
@@ -835,9 +1067,9 @@ __device__ __forceinline__ void kron3d_body(const KronParams<Real>& P) {
       for (int ch = lane; ch < nchunks; ch += 32) {
         const int d = ch * S::CR;
         const int r = d / NNN, o = d - r * NNN;
-        const int z = o / NN, w = o - z * NN;
+        const int z = o / NN, q0 = o - z * NN;
         Real v[S::CR];
-        vload<Real, S::CR>(buf + r * S::SE + z * S::SP + w, v);
+        vload<Real, S::CR>(buf + r * S::SE + z * S::SP + q0, v);
         if (by == Real(0)) {
 #pragma unroll
           for (int q = 0; q < S::CR; ++q) v[q] = alpha * v[q];
@@ -876,16 +1108,31 @@ __device__ __forceinline__ void kron3d_body(const KronParams<Real>& P) {
   }
 }
 
-template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime>
-__global__ void __launch_bounds__(128) kron3d_kernel(const __grid_constant__ KronParams<Real> P) {
-  kron3d_body<N, Real, SEP, STAGES, SHFL, DOT, VM>(P);
+// CTAs of 128 threads per SM the register allocation aims at: planes X and out and a few lines
+// live at once.
+template <int N, typename Real>
+constexpr int kron3d_min_ctas() {
+  return sizeof(Real) == 8 ? (N <= 4 ? 4 : (N == 5 ? 3 : 2)) : (N <= 4 ? 6 : 4);
 }
 
-// The FP64 slot-mask forms without a separate mass term, held to the run-time form's 4 CTAs per
-// SM (at most 128 registers; left to itself the compiler takes 138 for kVarySheared).
-template <int N, int STAGES, bool SHFL, bool DOT, uint32_t VM>
-__global__ void __launch_bounds__(128, 4) kron3d_kernel_capped(const __grid_constant__ KronParams<double> P) {
-  kron3d_body<N, double, false, STAGES, SHFL, DOT, VM>(P);
+template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime,
+          bool GEN = false>
+__global__ void __launch_bounds__(128, kron3d_min_ctas<N, Real>())
+    kron3d_kernel(const __grid_constant__ KronParams<Real> P) {
+  kron3d_body<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>(P);
+}
+
+// Face words of every element (P.eflags of later launches), for operators with advection terms:
+// words[e] of the forward operator, words[nelem + e] of the transposed one.
+template <typename Real>
+__global__ void kron_face_words(const KronParams<Real> fwd, const KronParams<Real> tr, uint32_t* words) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < fwd.nelem;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    uint32_t c[3];
+    kron_coords(fwd, (uint32_t)e, c);
+    words[e] = face_word(fwd, e, c);
+    words[fwd.nelem + e] = face_word(tr, e, c);
+  }
 }
 
 }  // namespace dgop

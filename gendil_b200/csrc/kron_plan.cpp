@@ -126,17 +126,21 @@ bool invert_table(std::vector<double>& mats, const KronMat& m, int64_t count, in
 
 // The Kronecker form for any dimension (see kron.h): eligibility of the coefficients and the
 // per-axis matrix tables.  Dimension- and size-specific limits are the callers'.
-KronPlanHost plan_kron(const KronInputs& in) {
+// `general`: the caller's kernel also takes bases without nodes on the faces and a density that is
+// a sum of products (in.sigma_terms).  Operators without advection terms have no faces and take
+// any basis everywhere.
+KronPlanHost plan_kron(const KronInputs& in, bool general) {
   KronPlanHost p;
   p.N = in.N;
   p.dim = in.D;
   const int Dm = in.D;
-  if (!in.gll) {
+  const bool adv = (in.flags & kAdvCell) != 0;
+  const bool mass = (in.flags & kMass) != 0;
+  if (!in.gll && (in.inverse_mass || (adv && !general))) {
     p.why = "basis is not GLL";
     return p;
   }
-  const bool adv = (in.flags & kAdvCell) != 0;
-  const bool mass = (in.flags & kMass) != 0;
+  p.gl = !in.gll && adv;
   if (!adv && !mass) {
     p.why = "empty operator";
     return p;
@@ -151,7 +155,8 @@ KronPlanHost plan_kron(const KronInputs& in) {
         p.why = "velocity component is not a single separable product";
         return p;
       }
-  if (mass && !in.sigma.separable) {
+  const bool sum = mass && !in.sigma.separable && general && in.num_sigma_terms > 0 && !in.inverse_mass;
+  if (mass && !in.sigma.separable && !sum) {
     p.why = "density is not a single separable product";
     return p;
   }
@@ -164,7 +169,7 @@ KronPlanHost plan_kron(const KronInputs& in) {
   if (adv) {
     // the mass term merges into the last axis' term when its other factors equal that term's
     const SepCoef& bl = in.beta[last];
-    bool same = mass && !in.sigma.has_elem && !bl.has_elem;
+    bool same = mass && !sum && !in.sigma.has_elem && !bl.has_elem;
     for (int k = 0; k < last && same; ++k) same = in.sigma.tab[k] == bl.tab[k];
     p.mass_merged = same;
     for (int a = 0; a < Dm; ++a) {
@@ -193,7 +198,12 @@ KronPlanHost plan_kron(const KronInputs& in) {
         }
     }
   }
-  if (mass && !p.mass_merged) {
+  if (sum) {
+    p.nextra = in.num_sigma_terms;
+    for (int t = 0; t < p.nextra; ++t)
+      for (int k = 0; k < Dm; ++k)
+        p.extra[t][k] = add_mass(M, in, k, in.sigma_terms[t].tab[k], k == last ? in.sigma_terms[t].c * detJ : 1.0);
+  } else if (mass && !p.mass_merged) {
     const double s_m = in.sigma.c * detJ;
     p.MD = add_mass(M, in, last, in.sigma.tab[last], s_m);
     for (int k = 0; k < last; ++k) p.MT[k] = add_mass(M, in, k, in.sigma.tab[k], 1.0);
@@ -218,15 +228,15 @@ KronPlanHost plan_kron3d(const KronInputs& in) {
     p.why = "dimension != 3";
     return p;
   }
-  if (in.N > 4) {  // the FP64 register kernel spills above N = 4
-    p.why = "order above 3 (register kernel limit)";
+  if (in.N > kKronMaxN) {  // the FP64 register kernel spills above N = 6
+    p.why = "order above 5 (register kernel limit)";
     return p;
   }
   if ((uint64_t)in.sizes[0] * in.sizes[1] * in.sizes[2] >= (uint64_t(1) << 32)) {
     p.why = "more than 2^32 elements";
     return p;
   }
-  return plan_kron(in);
+  return plan_kron(in, true);
 }
 
 }  // namespace dgop

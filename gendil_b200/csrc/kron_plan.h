@@ -15,13 +15,17 @@ struct KronInputs {
   const double* Dq = nullptr;  // Q x Q
   const double* wq = nullptr;  // Q
   SepCoef sigma;
+  // the density as a sum of products, when it is not a single one (3D register kernel only)
+  const SepCoef* sigma_terms = nullptr;
+  int num_sigma_terms = 0;
   SepCoef beta[kMaxDim];
   bool inverse_mass = false;  // plan the inverse of the (mass-only) operator
 };
 
 // Any dimension (dimension- and size-specific limits are the callers').
-KronPlanHost plan_kron(const KronInputs& in);
-// The 3D register kernel's plan: D = 3, N <= 4, fewer than 2^32 elements.
+KronPlanHost plan_kron(const KronInputs& in, bool general = false);
+// The 3D register kernel's plan: D = 3, N <= kKronMaxN, fewer than 2^32 elements; also bases without
+// nodes on the faces and densities that are sums of products.
 KronPlanHost plan_kron3d(const KronInputs& in);
 
 }  // namespace dgop

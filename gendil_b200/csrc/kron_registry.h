@@ -34,6 +34,8 @@ struct KronVariant {
   // compile-time slot-mask forms of the above (one-stage tile variants): [mask index, kron.h]
   // [with the inner-product epilogue][separate mass term]
   const void* func_masked[2][2][2] = {};
+  // the general form (KronParams::general): [with the inner-product epilogue][separate mass term]
+  const void* func_general[2][2] = {};
   int warp_smem = 0;               // Real values of shared memory per warp (bytes per CTA for bulk-tensor variants)
   int threads = 0;                 // threads per CTA
 };
@@ -42,13 +44,19 @@ template <typename Real>
 struct KronEntry {
   int epw = 0;  // elements per warp group
   KronVariant<Real> v[kKronVariants];
-  // per-element face words / per-group slot words of the bulk-tensor variants
-  void (*face_words)(const KronParams<Real>& p, uint32_t* eflags, uint32_t* gwords, cudaStream_t s) = nullptr;
+  // face words of the forward and the transposed operator (KronParams::eflags), 2 nelem of them; the bulk-tensor variants' face and slot words
+  void (*face_words)(const KronParams<Real>& fwd, const KronParams<Real>& tr, uint32_t* words, cudaStream_t s) = nullptr;
+  void (*tma_words)(const KronParams<Real>& p, uint32_t* eflags, uint32_t* gwords, cudaStream_t s) = nullptr;
 };
 
 KronEntry<double>& kron3d_slot_f64(int N);
 KronEntry<float>& kron3d_slot_f32(int N);
-void register_kron3d();
+void register_kron3d_n1();
+void register_kron3d_n2();
+void register_kron3d_n3();
+void register_kron3d_n4();
+void register_kron3d_n5();
+void register_kron3d_n6();
 
 // Kronecker form, any dimension, shared-memory kernel (kronnd_kernel.cuh).  Variants (the
 // autotuner picks one per operator): 0 one shared-memory pass per axis; 1, 2 groups of 2 or 3

@@ -10,7 +10,7 @@
 
 namespace dgop {
 
-// Face word of an element (kron_face_words): per face f = 2 a + s, 5 bits: kRecCorner, kRecNb,
+// Face word of an element (kron_tma_words): per face f = 2 a + s, 5 bits: kRecCorner, kRecNb,
 // kRecG and the trace source in bits 3-4: 0 the group's own planes (x faces), 1 the group's
 // staged slice slot of that axis (for x: the neighbour element staged beside the group, in the
 // variants that stage it; the others read it from global memory), 2 global memory.

@@ -39,7 +39,12 @@ void ensure_registry() {
   DGOP_CALL_N(D, 1) DGOP_CALL_N(D, 2) DGOP_CALL_N(D, 3) DGOP_CALL_N(D, 4) \
   DGOP_CALL_N(D, 5) DGOP_CALL_N(D, 6) DGOP_CALL_N(D, 7) DGOP_CALL_N(D, 8)
     DGOP_CALL_D(1) DGOP_CALL_D(2) DGOP_CALL_D(3) DGOP_CALL_D(4) DGOP_CALL_D(5) DGOP_CALL_D(6)
-    register_kron3d();
+    register_kron3d_n1();
+    register_kron3d_n2();
+    register_kron3d_n3();
+    register_kron3d_n4();
+    register_kron3d_n5();
+    register_kron3d_n6();
     register_kronnd_d1();
     register_kronnd_d2();
     register_kronnd_d3();

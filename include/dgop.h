@@ -109,10 +109,11 @@ int64_t dgop_operator_num_dofs(const dgop_operator* op);
 /* Kernel family used by an operator (no reference counterpart; diagnostics and testing):
  * DGOP_KERNEL_GENERIC is the sum-factorized kernel that follows the reference's element
  * algorithm for every shape; DGOP_KERNEL_KRON is the register-resident Kronecker-form kernel
- * (3D, GLL, orders 0..3, separable coefficients), chosen automatically when eligible;
+ * (3D, orders 0..5, velocity components that are separable products; a density may be a sum of
+ * products), chosen automatically when eligible;
  * DGOP_KERNEL_KRONND is the shared-memory Kronecker-form kernel for any dimension and order
- * (GLL, separable coefficients, element within shared memory), chosen when the register kernel
- * does not apply.
+ * (separable coefficients, with advection terms the GLL basis, element within shared memory),
+ * chosen when the register kernel does not apply.
  * dgop_operator_kernel_note() says why the Kronecker form was not chosen. */
 enum dgop_kernel {
   DGOP_KERNEL_GENERIC = 0,
@@ -126,7 +127,8 @@ const char* dgop_operator_kernel_note(const dgop_operator* op);
 int dgop_operator_select_kernel(dgop_operator* op, int kernel);
 /* Kronecker-kernel variants (no reference counterpart): 0 "stage2-tile" (next element group staged
  * while this one computes, layout exchanges through shared memory), 1 "stage1-tile" (one staging
- * buffer, more warps per SM), 2 "stage2-shfl" (exchanges by warp shuffles; even orders), and for
+ * buffer, more warps per SM; the only one above order 3), 2 "stage2-shfl" (exchanges by warp
+ * shuffles; orders 1 and 3), and for
  * p = 3 FP64 operators whose x extent is a multiple of 8, element groups moved by the Tensor
  * Memory Accelerator: 3 "tma1-tile", 4 "tma2-shfl", 5 "tma2-tile".  At
  * creation the autotuner times every variant on scratch vectors (operators of at most 2^26 DoFs)

@@ -1,0 +1,100 @@
+"""GPU: the 3D register kernel over the orders and forms it takes (p = 0..5, bases without nodes on
+the faces, densities that are sums of products, per-element factors), against the oracle or the
+generic kernel."""
+import numpy as np
+import pytest
+import torch
+
+import gendil_b200 as g
+from gendil_b200 import coefficients as C
+from helpers import APPLY_TOL, cuda_apply, inputs, make_operator, oracle, rel_max
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(p, q, sizes, basis=0, beta=2, sigma=0, periodic=(0, 0, 0), gval=0.5, c=None):
+    return {"D": 3, "P": p, "Q": q, "basis": basis, "sizes": list(sizes), "h": [1.0 / n for n in sizes],
+            "origin": [0.0] * 3, "periodic": list(periodic), "beta_kind": beta, "beta_c": c, "sigma_kind": sigma,
+            "sigma_c": 2.0, "g": gval, "seed": 3}
+
+
+# element counts around the warp's group (32 / (p + 1) elements), inflow on either or both sides of
+# an axis, wrapped neighbours inside and outside the group, varying and constant matrices
+CASES = ([("p%d" % p, _case(p, p + 2, (7, 3, 5))) for p in range(6)] +
+         [("p%d_bubble" % p, _case(p, p + 1, (32 // (p + 1) + 1, 2, 3), beta=1)) for p in (1, 4, 5)] +
+         [("p%d_wrap" % p, _case(p, p + 1, (5, 4, 3), beta=0, c=[-0.7, 0.4, -0.3], periodic=(1, 1, 1)))
+          for p in (2, 4, 5)] +
+         [("gl%d" % p, _case(p, p + 1, (6, 5, 4), basis=1, beta=b)) for p, b in ((0, 0), (1, 1), (2, 2), (3, 1), (4, 1), (5, 2))] +
+         [("gl3_wrap", _case(3, 5, (9, 3, 2), basis=1, beta=0, c=[0.6, -0.2, 0.5], periodic=(1, 0, 1)))] +
+         [("poly%d" % p, _case(p, p + 1, (6, 3, 7), sigma=1)) for p in (1, 3, 4, 5)] +
+         [("gl2_poly", _case(2, 4, (5, 4, 3), basis=1, beta=1, sigma=1))])
+for _, _c in CASES:
+    if _c["beta_kind"] == 0 and _c["beta_c"] is None:
+        _c["beta_c"] = [0.7, -0.4, 0.25]
+
+
+@pytest.mark.parametrize("case", [c for _, c in CASES], ids=[n for n, _ in CASES])
+def test_register_kernel_matches_oracle_and_generic(case):
+    x = inputs(case)
+    for kind, mode in (("mass", 1), ("adv", 0), ("adv", 1), ("adv", 2)):
+        op = make_operator(case, kind, mode)
+        assert op.kernel == "kron", op.kernel_note
+        want = oracle().mass_apply(case, x) if kind == "mass" else oracle().advection_apply(case, x, mode)
+        y = cuda_apply(op, x)
+        assert rel_max(y, want) <= APPLY_TOL, (kind, mode)
+        yt, y32 = cuda_apply(op, x, transpose=True), cuda_apply(op, x, f32=True)
+        xd = torch.from_numpy(x).cuda()
+        yb = torch.from_numpy(x[::-1].copy()).cuda()
+        op.apply(xd, yb, alpha=2.5, beta=-0.5)
+        assert rel_max(yb.cpu().numpy(), 2.5 * y - 0.5 * x[::-1]) <= 1e-14
+        try:
+            op.select_kernel("generic")
+        except g.DGOPError:
+            continue  # no generic kernel for this shape
+        assert rel_max(yt, cuda_apply(op, x, transpose=True)) <= APPLY_TOL, (kind, mode)
+        # FP32: each of the three contractions rounds sums of N (N + 1) / 2-term products; 1e-5 of
+        # the largest value as for the other FP32 applies
+        assert rel_max(y32, y) <= 1e-5, (kind, mode)
+
+
+@pytest.mark.parametrize("basis", [g.GLL, g.GL])
+@pytest.mark.parametrize("p", [2, 3, 5])
+def test_per_element_factors_are_read_at_every_apply(p, basis):
+    """Velocity factors changed in place (signs included) between applies: the upwind decisions
+    follow the new values, as on the generic kernel."""
+    sp = g.Space(3, [8, 3, 4], order=p, basis=basis)
+    rng = np.random.default_rng(1)
+    factor = torch.from_numpy(rng.uniform(0.5, 1.5, sp.num_elements)).cuda()
+    beta = [C.Coefficient(constant=v, element_factor=factor) for v in (0.8, -0.5, 0.3)]
+    op = g.SystemOperator(sp, p + 1, beta, sigma=C.Coefficient(constant=3.0, element_factor=factor))
+    gen = g.SystemOperator(sp, p + 1, beta, sigma=C.Coefficient(constant=3.0, element_factor=factor))
+    assert op.kernel == "kron", op.kernel_note
+    gen.select_kernel("generic")
+    x = rng.uniform(-1, 1, sp.num_dofs)
+    for _ in range(2):
+        for tr in (False, True):
+            assert rel_max(cuda_apply(op, x, transpose=tr), cuda_apply(gen, x, transpose=tr)) <= APPLY_TOL
+        factor.mul_(torch.from_numpy(rng.choice([-1.0, 1.0], sp.num_elements)).cuda())
+
+
+def test_sums_that_are_one_product_are_merged():
+    """A constant plus functions of one coordinate is one separable product: such velocities and
+    densities take the Kronecker kernels in every dimension, with the generic kernel's results."""
+    for D, sizes in ((2, [5, 7]), (3, [5, 4, 3])):
+        sp = g.Space(D, sizes, order=3)
+        beta = [C.Coefficient(constant=1.0, terms=[{(a + 1) % D: lambda x: 0.5 * x * x}, {(a + 1) % D: lambda x: 0.2 * x}])
+                for a in range(D)]
+        op = g.SystemOperator(sp, 5, beta, sigma=C.Coefficient(constant=2.0, terms=[{0: lambda x: x}]))
+        assert op.kernel == ("kronnd" if D == 2 else "kron"), op.kernel_note
+        x = np.random.default_rng(0).uniform(-1, 1, sp.num_dofs)
+        y = cuda_apply(op, x)
+        op.select_kernel("generic")
+        assert rel_max(y, cuda_apply(op, x)) <= APPLY_TOL
+
+
+def test_mass_inverse_stays_limited_to_single_products():
+    sp = g.Space(3, [3, 3, 3], order=2)
+    with pytest.raises(g.DGOPError):
+        g.MassInverseOperator(sp, 4, C.Coefficient(constant=1.0, terms=[{0: lambda x: x}]))
+    with pytest.raises(g.DGOPError):
+        g.MassInverseOperator(g.Space(3, [3, 3, 3], order=2, basis=g.GL), 4, 1.0)
