@@ -607,7 +607,8 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     if (!kv.launch && !(kv.launch_tma && tma_shape)) continue;
     const int threads = kv.threads, warps = threads / 32;
     L.block = dim3(threads);
-    L.smem = kv.launch_tma ? (size_t)kv.warp_smem : (size_t)warps * kv.warp_smem * sizeof(Real);
+    L.smem = kv.launch_tma ? (size_t)kv.warp_smem
+                           : (size_t)warps * (p.general ? kv.warp_smem_general : kv.warp_smem) * sizeof(Real);
     if ((int)L.smem > max_smem - 1024) continue;  // 1 KB covers every variant's static shared memory
     int arc = allow_dynamic_smem(kv.func, max_smem);
     if (arc == DGOP_OK) arc = allow_dynamic_smem(kv.func_sep, max_smem);

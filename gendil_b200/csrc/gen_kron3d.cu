@@ -1,6 +1,7 @@
 // Instantiations of the 3D Kronecker-form kernel, FP64 and FP32, every variant; compiled once per
 // order with -DDGOP_GEN_N=<p + 1>, N = 1..6.
 #include "kron3d_kernel.cuh"
+#include "kron3d_p3_kernel.cuh"
 #include "kron3d_tma_kernel.cuh"
 #include "kron_registry.h"
 
@@ -32,20 +33,31 @@ constexpr bool masked_forms() {
   return N >= 4 && STAGES == 1 && !SHFL;
 }
 
+// The kernel of a variant: FP64 N = 4 has its own schedule (kron3d_p3_kernel.cuh).
+template <int N, typename Real>
+constexpr bool own_schedule() {
+  return N == 4 && std::is_same<Real, double>::value;
+}
+template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false>
+constexpr auto kernel_entry() {
+  if constexpr (own_schedule<N, Real>() && !GEN) return &kron3d_p3_kernel<SEP, STAGES, SHFL, DOT, VM>;
+  else return &kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>;
+}
+
 template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT>
 void launch_kron3d_masked(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
   if constexpr (masked_forms<N, STAGES, SHFL>()) {
     const int mi = kron_mask_index(p);
     if (mi == 0) {
-      kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, kVaryNone><<<grid, block, smem, s>>>(p);
+      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryNone>()<<<grid, block, smem, s>>>(p);
       return;
     }
     if (mi == 1) {
-      kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, kVarySheared><<<grid, block, smem, s>>>(p);
+      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVarySheared>()<<<grid, block, smem, s>>>(p);
       return;
     }
   }
-  kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT><<<grid, block, smem, s>>>(p);
+  kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryRuntime>()<<<grid, block, smem, s>>>(p);
 }
 
 template <int N, typename Real, int STAGES, bool SHFL>
@@ -76,7 +88,7 @@ void launch_kron3d(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem
 
 template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false>
 const void* kernel_of() {
-  return reinterpret_cast<const void*>(&kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>);
+  return reinterpret_cast<const void*>(kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, VM, GEN>());
 }
 
 template <int N, typename Real, int STAGES, bool SHFL>
@@ -106,7 +118,8 @@ void fill_variant(KronVariant<Real>& v) {
     v.func_general[1][0] = kernel_of<N, Real, STAGES, SHFL, false, true, kVaryRuntime, true>();
     v.func_general[1][1] = kernel_of<N, Real, STAGES, SHFL, true, true, kVaryRuntime, true>();
   }
-  v.warp_smem = Kron3DShape<N, Real>::warp_smem(STAGES, SHFL);
+  v.warp_smem_general = Kron3DShape<N, Real>::warp_smem(STAGES, SHFL);
+  v.warp_smem = own_schedule<N, Real>() ? KronP3Shape<N, Real>::warp_smem(STAGES, SHFL) : v.warp_smem_general;
   v.threads = kKronThreads;
 }
 

@@ -37,6 +37,7 @@ struct KronVariant {
   // the general form (KronParams::general): [with the inner-product epilogue][separate mass term]
   const void* func_general[2][2] = {};
   int warp_smem = 0;               // Real values of shared memory per warp (bytes per CTA for bulk-tensor variants)
+  int warp_smem_general = 0;       // Real values per warp of the general form
   int threads = 0;                 // threads per CTA
 };
 
