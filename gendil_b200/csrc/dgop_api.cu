@@ -1403,7 +1403,34 @@ static int launch_impl(dgop_operator* op, LaunchCfg<Real>& L, KronCfg<Real>& K, 
       set_error("the transposed interior-penalty operator is provided for the symmetric form (sigma = -1) only");
       return DGOP_ERR_UNSUPPORTED;
     }
-    KronDiffParams<Real> p = SD.params;  // symmetric for sigma = -1: the transpose is the operator
+    if (SD.entry3d && aligned16) {
+      Kron3DDiffParams<Real> p = SD.params3d;  // symmetric for sigma = -1: the transpose is the operator
+      p.x = x;
+      p.y = y;
+      p.alpha = alpha;
+      p.beta_y = beta_y;
+      p.skip = skip;
+      p.e_begin = e_begin;
+      p.nelem = e_end;
+      p.dot_z = nullptr;
+      p.dot_partials = nullptr;
+      p.dot_count = 0;
+      dim3 grid = SD.grid3d[0];
+      if constexpr (sizeof(Real) == 8) {
+        if (dot && dot->z && dot->partials && reinterpret_cast<uintptr_t>(dot->z) % 16 == 0 && dot->count > 0) {
+          p.dot_z = dot->z;
+          p.dot_partials = dot->partials;
+          p.dot_count = dot->count;
+          grid.x = std::min<unsigned>(SD.grid3d[1].x, (unsigned)dot->count);
+          if (dot->fused) *dot->fused = true;
+        }
+      }
+      SD.entry3d->launch_diff(p, SD.gll, grid, SD.block3d, SD.smem3d, s);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return cuda_fail(e, "operator kernel launch");
+      return DGOP_OK;
+    }
+    KronDiffParams<Real> p = SD.params;
     p.x = x;
     p.y = y;
     p.alpha = alpha;

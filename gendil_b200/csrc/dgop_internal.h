@@ -112,6 +112,12 @@ struct KronDiffCfg {
   size_t smem = 0;
   Real* d_mats = nullptr;
   Real* d_mu = nullptr;  // FP32 copy of the per-element diffusivity
+  // 3D register kernel (orders 1..5; 16-byte aligned vectors), plain and with the inner-product epilogue
+  const KronEntry<Real>* entry3d = nullptr;
+  Kron3DDiffParams<Real> params3d{};
+  bool gll = true;
+  dim3 grid3d[3], block3d;  // grids by DiffMode: apply, apply with the epilogue, coefficient gradient
+  size_t smem3d = 0, smem3d_grad = 0;
   // coefficient-gradient kernel launch (FP64)
   bool grad_ready = false;
   int grad_eb = 0;

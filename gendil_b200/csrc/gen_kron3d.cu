@@ -1,5 +1,6 @@
 // Instantiations of the 3D Kronecker-form kernel, FP64 and FP32, every variant; compiled once per
 // order with -DDGOP_GEN_N=<p + 1>, N = 1..6.
+#include "kron3d_diff_kernel.cuh"
 #include "kron3d_kernel.cuh"
 #include "kron3d_p3_kernel.cuh"
 #include "kron3d_tma_kernel.cuh"
@@ -173,6 +174,24 @@ void fill_tma(KronVariant<double>& v) {
   v.threads = kTmaWarps * 32;
 }
 
+template <int N, typename Real>
+void launch_diff(const Kron3DDiffParams<Real>& p, bool gll, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+  if constexpr (std::is_same<Real, double>::value) {
+    if (p.gout) {
+      if (gll) kron3d_diff_kernel<N, Real, true, kDiffGradient><<<grid, block, smem, s>>>(p);
+      else kron3d_diff_kernel<N, Real, false, kDiffGradient><<<grid, block, smem, s>>>(p);
+      return;
+    }
+    if (p.dot_partials) {
+      if (gll) kron3d_diff_kernel<N, Real, true, kDiffApplyDot><<<grid, block, smem, s>>>(p);
+      else kron3d_diff_kernel<N, Real, false, kDiffApplyDot><<<grid, block, smem, s>>>(p);
+      return;
+    }
+  }
+  if (gll) kron3d_diff_kernel<N, Real, true, kDiffApply><<<grid, block, smem, s>>>(p);
+  else kron3d_diff_kernel<N, Real, false, kDiffApply><<<grid, block, smem, s>>>(p);
+}
+
 template <typename Real>
 void face_words(const KronParams<Real>& fwd, const KronParams<Real>& tr, uint32_t* words, cudaStream_t s) {
   const int64_t blocks = std::min<int64_t>((fwd.nelem + 255) / 256, 4096);
@@ -193,6 +212,19 @@ void fill(KronEntry<Real>& d) {
   fill_variant<N, Real, 1, false>(d.v[1]);
   if constexpr (Kron3DShape<N, Real>::BUTTERFLY) fill_variant<N, Real, 2, true>(d.v[2]);
   d.face_words = &face_words<Real>;
+  if constexpr (N >= 2) {
+    d.launch_diff = &launch_diff<N, Real>;
+    d.func_diff[0][kDiffApply] = reinterpret_cast<const void*>(&kron3d_diff_kernel<N, Real, false, kDiffApply>);
+    d.func_diff[1][kDiffApply] = reinterpret_cast<const void*>(&kron3d_diff_kernel<N, Real, true, kDiffApply>);
+    if constexpr (std::is_same<Real, double>::value) {
+      d.func_diff[0][kDiffApplyDot] = reinterpret_cast<const void*>(&kron3d_diff_kernel<N, Real, false, kDiffApplyDot>);
+      d.func_diff[1][kDiffApplyDot] = reinterpret_cast<const void*>(&kron3d_diff_kernel<N, Real, true, kDiffApplyDot>);
+      d.func_diff[0][kDiffGradient] = reinterpret_cast<const void*>(&kron3d_diff_kernel<N, Real, false, kDiffGradient>);
+      d.func_diff[1][kDiffGradient] = reinterpret_cast<const void*>(&kron3d_diff_kernel<N, Real, true, kDiffGradient>);
+    }
+    d.diff_warp_smem[0] = Kron3DDiffShape<N, Real>::WARP;
+    d.diff_warp_smem[1] = Kron3DDiffShape<N, Real, true>::WARP;
+  }
 #if DGOP_GEN_N == 4
   if constexpr (std::is_same<Real, double>::value) {
     fill_tma<1, false>(d.v[3]);

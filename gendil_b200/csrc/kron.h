@@ -193,6 +193,32 @@ struct KronDiffParams {
   Real face_h[kMaxDim];  // detJ / h_a^2
 };
 
+// The 3D register kernel of the diffusion operator (kron3d_diff_kernel.cuh, sipdg.cu).
+template <typename Real>
+struct Kron3DDiffParams {
+  int64_t nelem, e_begin;  // elements [e_begin, nelem), fewer than 2^32
+  FastDiv fdx, fdy;        // element index -> coordinates
+  int64_t sizes[3];
+  int periodic[3];
+  int boundary;
+  Real sigma, kappa, alpha, beta_y;
+  Real f[3];               // detJ / h_a^2
+  const Real* x;
+  Real* y;
+  const Real* mu;
+  const int* skip;
+  Real kint[3][kKronMaxN * kKronMaxN];  // Khat_a and the own face terms of an element between others
+  Real mm[3][kKronMaxN * kKronMaxN];    // 1D mass matrices
+  Real tv[4][kKronMaxN];                // l(0), l(1), l'(0), l'(1)
+  const Real* dot_z;       // optional epilogue, as in KronParams
+  double* dot_partials;
+  int dot_count;
+  // coefficient gradient: gout[e] = gscale[e] lam^T (dA/dmu_e) x
+  const Real* lam;
+  Real* gout;
+  const Real* gscale;
+};
+
 struct KronPlanHost {
   bool ok = false;
   const char* why = "";

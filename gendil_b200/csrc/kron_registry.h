@@ -45,6 +45,13 @@ template <typename Real>
 struct KronEntry {
   int epw = 0;  // elements per warp group
   KronVariant<Real> v[kKronVariants];
+  // interior-penalty diffusion (kron3d_diff_kernel.cuh): [basis with nodes on the faces][DiffMode]
+  // (the apply; FP64 also with the inner-product epilogue, and the coefficient gradient), shared
+  // memory per warp in Reals [gradient]
+  void (*launch_diff)(const Kron3DDiffParams<Real>& p, bool gll, dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t s) = nullptr;
+  const void* func_diff[2][3] = {};
+  int diff_warp_smem[2] = {};
   // face words of the forward and the transposed operator (KronParams::eflags), 2 nelem of them; the bulk-tensor variants' face and slot words
   void (*face_words)(const KronParams<Real>& fwd, const KronParams<Real>& tr, uint32_t* words, cudaStream_t s) = nullptr;
   void (*tma_words)(const KronParams<Real>& p, uint32_t* eflags, uint32_t* gwords, cudaStream_t s) = nullptr;

@@ -121,6 +121,70 @@ int setup_grad(dgop_operator* op, KronDiffCfg<double>& K) {
   return DGOP_OK;
 }
 
+// The 3D register kernel's launch (kron3d_diff_kernel.cuh), where it covers the order; leaves entry3d
+// null otherwise.
+template <typename Real>
+int setup_diff3d(dgop_operator* op, KronDiffCfg<Real>& K, const std::vector<double>& mats, double sigma, double kappa) {
+  const dgop_space& s = op->sp;
+  const int N = s.n;
+  if (s.D != 3 || N < 2 || N > kKronMaxN || s.nelem >= (int64_t(1) << 32)) return DGOP_OK;
+  const KronEntry<Real>* entry = nullptr;
+  if constexpr (sizeof(Real) == 8) entry = &kron3d_slot_f64(N);
+  else entry = &kron3d_slot_f32(N);
+  if (!entry->launch_diff) return DGOP_OK;
+  Kron3DDiffParams<Real>& p = K.params3d;
+  std::memset(&p, 0, sizeof(p));
+  p.nelem = s.nelem;
+  p.fdx = FastDiv((uint32_t)s.sizes[0]);
+  p.fdy = FastDiv((uint32_t)s.sizes[1]);
+  const double* tv = mats.data() + (size_t)3 * kDiffMats * N * N;
+  for (int k = 0; k < 4; ++k)
+    for (int i = 0; i < N; ++i) p.tv[k][i] = (Real)tv[k * N + i];
+  for (int a = 0; a < 3; ++a) {
+    p.sizes[a] = s.sizes[a];
+    p.periodic[a] = s.periodic[a];
+    p.f[a] = K.params.face_h[a];
+    const double f = s.h[0] * s.h[1] * s.h[2] / (s.h[a] * s.h[a]);
+    for (int i = 0; i < N; ++i)
+      for (int j = 0; j < N; ++j) {
+        double v = mats[((size_t)a * kDiffMats + kDK) * N * N + i * N + j];
+        for (int side = 0; side < 2; ++side) {
+          const double nu = side ? 1.0 : -1.0;
+          const double *b = tv + side * N, *d = tv + (2 + side) * N;
+          v += f * (-0.5 * nu * b[i] * d[j] + 0.5 * kappa * b[i] * b[j] + 0.5 * sigma * nu * d[i] * b[j]);
+        }
+        p.kint[a][i * N + j] = (Real)v;
+        p.mm[a][i * N + j] = (Real)mats[((size_t)a * kDiffMats + kDM) * N * N + i * N + j];
+      }
+  }
+  p.boundary = K.params.boundary;
+  p.sigma = K.params.sigma;
+  p.kappa = K.params.kappa;
+  p.mu = K.params.mu;
+  K.gll = s.basis == DGOP_BASIS_GLL;
+  // small meshes: fewer warps per CTA, so that every SM gets some
+  const int64_t groups = (s.nelem + entry->epw - 1) / entry->epw, sms = device_sms(op->device);
+  const int warps = groups <= 4 * sms ? 1 : (groups <= 8 * sms ? 2 : 4);
+  K.block3d = dim3(32 * warps);
+  K.smem3d = (size_t)warps * entry->diff_warp_smem[0] * sizeof(Real);
+  K.smem3d_grad = (size_t)warps * entry->diff_warp_smem[1] * sizeof(Real);
+  int max_smem = 0;
+  DGOP_CUDA_D(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, op->device));
+  if (K.smem3d_grad + 1024 > (size_t)max_smem) return DGOP_OK;
+  for (int mode = 0; mode < 3; ++mode) {
+    const void* f = entry->func_diff[K.gll ? 1 : 0][mode];
+    if (!f) continue;
+    DGOP_CUDA_D(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - 1024));
+    int per_sm = 0;
+    DGOP_CUDA_D(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 32 * warps,
+                                                              mode == 2 ? K.smem3d_grad : K.smem3d));
+    if (per_sm < 1) return DGOP_OK;
+    K.grid3d[mode] = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((groups + warps - 1) / warps, sms * per_sm)));
+  }
+  K.entry3d = entry;
+  return DGOP_OK;
+}
+
 template <typename Real>
 int setup_diff(dgop_operator* op, KronDiffCfg<Real>& K, const std::vector<double>& mats, const double* mu,
                double sigma, double kappa, int boundary) {
@@ -163,6 +227,8 @@ int setup_diff(dgop_operator* op, KronDiffCfg<Real>& K, const std::vector<double
     DGOP_CUDA_D(cudaGetLastError());
     p.mu = K.d_mu;
   }
+  const int rc3 = setup_diff3d<Real>(op, K, mats, sigma, kappa);
+  if (rc3 != DGOP_OK) return rc3;
   // elements per CTA: as many as fit in ~72 KB (three CTAs per SM), then, among the counts down
   // to half of that, the one whose lines fill the CTA's passes best (every pass runs over the
   // lines of all the CTA's elements, kKronNDThreads at a time)
@@ -271,6 +337,17 @@ extern "C" int dgop_sipdg_gradient(const dgop_operator* op, const double* u, con
   if (!K.grad_ready) {
     set_error("no coefficient-gradient kernel for this (dimension, order): the element exceeds shared memory");
     return DGOP_ERR_UNSUPPORTED;
+  }
+  if (K.entry3d && reinterpret_cast<uintptr_t>(u) % 16 == 0) {
+    Kron3DDiffParams<double> p = K.params3d;
+    p.x = u;
+    p.lam = lambda;
+    p.gout = out;
+    p.gscale = scale;
+    K.entry3d->launch_diff(p, K.gll, K.grid3d[2], K.block3d, K.smem3d_grad, (cudaStream_t)stream);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return cuda_fail(e, "coefficient-gradient kernel launch");
+    return DGOP_OK;
   }
   KronDiffParams<double> p = K.params;
   p.x = u;
