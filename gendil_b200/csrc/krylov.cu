@@ -151,15 +151,32 @@ __global__ void __launch_bounds__(kRT) k_cg_init_p(const CGState* st, const doub
 // of the solve (kCheckEvery is even, so the parity of the two agrees).
 
 // alpha = (r, r) / (p, A p); x += alpha p; r -= alpha A p; partials2 <- |r|^2   (:176-181)
+// (The first values of each thread are loaded before the sum of the partials: on small systems,
+// where a thread has no others, the two latencies overlap.)
 __global__ void __launch_bounds__(kRT) k_cg_update(int kk, const CGState* st, double* __restrict__ x,
                                                    double* __restrict__ r, const double* __restrict__ p,
                                                    const double* __restrict__ ap, int64_t n, const double* partials1,
                                                    double* partials2) {
+  const int64_t i0 = blockIdx.x * (int64_t)kRT + threadIdx.x;
+  double x0 = 0.0, r0 = 0.0, p0 = 0.0, a0 = 0.0;
+  if (i0 < n) {
+    x0 = x[i0];
+    r0 = r[i0];
+    p0 = p[i0];
+    a0 = ap[i0];
+  }
+  const double pap = reduce_partials(partials1);
   if (st->done) return;
   const int k = st->base + kk;
-  const double alpha = st->abs_[k & 1] / reduce_partials(partials1);
+  const double alpha = st->abs_[k & 1] / pap;
   double v = 0.0;
-  DGOP_GRID_LOOP(i, n) {
+  if (i0 < n) {
+    x[i0] = x0 + alpha * p0;
+    const double ri = r0 + (-alpha) * a0;
+    r[i0] = ri;
+    v += ri * ri;
+  }
+  for (int64_t i = i0 + (int64_t)kRB * kRT; i < n; i += (int64_t)kRB * kRT) {
     x[i] = x[i] + alpha * p[i];
     const double ri = r[i] + (-alpha) * ap[i];
     r[i] = ri;
@@ -171,11 +188,17 @@ __global__ void __launch_bounds__(kRT) k_cg_update(int kk, const CGState* st, do
 // stopping test, beta = (r_new, r_new) / (r_old, r_old), p = beta p + r   (:183-205)
 __global__ void __launch_bounds__(kRT) k_cg_finish(int kk, CGState* st, const double* __restrict__ r,
                                                    double* __restrict__ p, int64_t n, const double* partials2) {
+  const int64_t i0 = blockIdx.x * (int64_t)kRT + threadIdx.x;
+  double r0 = 0.0, p0 = 0.0;
+  if (i0 < n) {
+    r0 = r[i0];
+    p0 = p[i0];
+  }
+  const double R = reduce_partials(partials2);
   if (st->done) return;
   const int k = st->base + kk;
   const double tol = st->tol;
   const int max_iters = st->max_iters;
-  const double R = reduce_partials(partials2);
   const double r_n = sqrt(R);
   const double rhs_n = st->rhs_n;
   if (r_n < tol * rhs_n) {
@@ -189,7 +212,8 @@ __global__ void __launch_bounds__(kRT) k_cg_finish(int kk, CGState* st, const do
     return;
   }
   const double beta = R / st->abs_[k & 1];
-  DGOP_GRID_LOOP(i, n) p[i] = p[i] * beta + r[i];
+  if (i0 < n) p[i0] = p0 * beta + r0;
+  for (int64_t i = i0 + (int64_t)kRB * kRT; i < n; i += (int64_t)kRB * kRT) p[i] = p[i] * beta + r[i];
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     st->abs_[(k + 1) & 1] = R;
     st->r_n = r_n;
@@ -276,22 +300,9 @@ __global__ void k_gm_backsub(const GMState* st, const double* H, const double* e
   gm_backsub(st, H, e1, y, m);
 }
 
-// x += y_i V_i for i < k, in order (the reference's sequence of Axpy calls, gmres.hpp:263-267)
-template <typename T>
-__global__ void __launch_bounds__(kRT) k_gm_update(const GMState* st, double* __restrict__ x,
-                                                   const T* __restrict__ V, int64_t ld, const double* y, int64_t n) {
-  if (st->done || st->k == 0) return;
-  const int k = st->k;
-  DGOP_GRID_LOOP(l, n) {
-    double xl = x[l];
-    for (int i = 0; i < k; ++i) xl = xl + y[i] * (double)V[(int64_t)i * ld + l];
-    x[l] = xl;
-  }
-}
-
 // ---------------------------------------------- GMRES with iterative refinement (inner basis)
 
-constexpr int kGsChunk = 8;     // basis vectors per block row of the projection pass
+constexpr int kGsChunk = 16;    // basis vectors per block row of the projection pass
 constexpr int kGsMaxRestart = 1000;
 
 template <typename T>
@@ -307,39 +318,88 @@ struct Vec16<double> {
   static constexpr int L = 2;
 };
 
-// wide[i * kRB + block] <- partial (V_i, w) for i <= j (blockIdx.y selects kGsChunk vectors);
-// 128-bit accesses over the padded stride, products and sums in FP64
+// x += y_i V_i for i < k, in order (the reference's sequence of Axpy calls, gmres.hpp:263-267):
+// 16-byte loads of the basis, eight vectors in flight per thread.  HBM-bound: 0.32 ms for 26 vectors of
+// 16.8 M FP32 values (6.0 TB/s with x), 0.98 ms with one 4-byte load at a time.
 template <typename T>
-__global__ void __launch_bounds__(kRT) k_gs_dots(const GMState* st, const T* __restrict__ V, int64_t ld, int j,
-                                                 const T* __restrict__ w, double* wide) {
-  if (st->inactive) return;
+__global__ void __launch_bounds__(kRT) k_gm_update(const GMState* st, double* __restrict__ x,
+                                                   const T* __restrict__ V, int64_t ld, const double* y, int64_t n) {
+  if (st->done || st->k == 0) return;
+  using V16 = typename Vec16<T>::type;
+  constexpr int L = Vec16<T>::L, U = 8;
+  const int k = st->k;
+  const int64_t ldv = ld / L;
+  const V16* v16 = reinterpret_cast<const V16*>(V);
+  DGOP_GRID_LOOP(u, (n + L - 1) / L) {
+    double a[L];
+#pragma unroll
+    for (int c = 0; c < L; ++c) a[c] = u * L + c < n ? x[u * L + c] : 0.0;
+    for (int i = 0; i < k; i += U) {
+      V16 w[U];
+#pragma unroll
+      for (int j = 0; j < U; ++j)
+        if (i + j < k) w[j] = v16[(int64_t)(i + j) * ldv + u];
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        if (i + j >= k) break;
+        T vv[L];
+        *reinterpret_cast<V16*>(vv) = w[j];
+        const double yi = y[i + j];
+#pragma unroll
+        for (int c = 0; c < L; ++c) a[c] = a[c] + yi * (double)vv[c];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < L; ++c)
+      if (u * L + c < n) x[u * L + c] = a[c];
+  }
+}
+
+// wide[i * kRB + block] <- partial (V_i, w) for i <= j (blockIdx.y selects kGsChunk vectors);
+// 128-bit accesses over the padded stride, products and sums in FP64.  HBM-bound; compiled per
+// number of vectors, so that a thread's loads are all in flight together: 167 us for 14 vectors of
+// 16.8 M FP32 values, 6.0 TB/s (a loop of conditional loads, eight vectors per block row: 222 us).
+template <int C, typename T>
+__device__ __forceinline__ void gs_dots(const T* __restrict__ V, int64_t ld, const T* __restrict__ w, int i0,
+                                        double* wide) {
   using V16 = typename Vec16<T>::type;
   constexpr int L = Vec16<T>::L;
-  const int i0 = blockIdx.y * kGsChunk;
-  const int cnt = min(kGsChunk, j + 1 - i0);
-  double acc[kGsChunk];
+  double acc[C];
 #pragma unroll
-  for (int c = 0; c < kGsChunk; ++c) acc[c] = 0.0;
-  const int64_t nv = ld / L;
+  for (int c = 0; c < C; ++c) acc[c] = 0.0;
+  const int64_t nv = ld / L, ldv = ld / L;
   const V16* w16 = reinterpret_cast<const V16*>(w);
   const V16* v16 = reinterpret_cast<const V16*>(V + (int64_t)i0 * ld);
-  const int64_t ldv = ld / L;
   DGOP_GRID_LOOP(u, nv) {
+    V16 x[C];
+    const V16 wx = w16[u];
+#pragma unroll
+    for (int c = 0; c < C; ++c) x[c] = v16[c * ldv + u];
     T wv[L];
-    *reinterpret_cast<V16*>(wv) = w16[u];
+    *reinterpret_cast<V16*>(wv) = wx;
 #pragma unroll
-    for (int c = 0; c < kGsChunk; ++c) {
-      if (c < cnt) {
-        T vv[L];
-        *reinterpret_cast<V16*>(vv) = v16[c * ldv + u];
+    for (int c = 0; c < C; ++c) {
+      T vv[L];
+      *reinterpret_cast<V16*>(vv) = x[c];
 #pragma unroll
-        for (int k = 0; k < L; ++k) acc[c] += (double)vv[k] * (double)wv[k];
-      }
+      for (int k = 0; k < L; ++k) acc[c] += (double)vv[k] * (double)wv[k];
     }
   }
 #pragma unroll
-  for (int c = 0; c < kGsChunk; ++c)
-    if (c < cnt) write_partial(wide + (int64_t)(i0 + c) * kRB, acc[c]);
+  for (int c = 0; c < C; ++c) write_partial(wide + (int64_t)(i0 + c) * kRB, acc[c]);
+}
+template <typename T>
+__global__ void __launch_bounds__(kRT, 2) k_gs_dots(const GMState* st, const T* __restrict__ V, int64_t ld, int j,
+                                                    const T* __restrict__ w, double* wide) {
+  if (st->inactive) return;
+  const int i0 = blockIdx.y * kGsChunk;
+  switch (min(kGsChunk, j + 1 - i0)) {
+#define DGOP_GS_CASE(C) case C: gs_dots<C>(V, ld, w, i0, wide); break;
+    DGOP_GS_CASE(1) DGOP_GS_CASE(2) DGOP_GS_CASE(3) DGOP_GS_CASE(4) DGOP_GS_CASE(5) DGOP_GS_CASE(6)
+    DGOP_GS_CASE(7) DGOP_GS_CASE(8) DGOP_GS_CASE(9) DGOP_GS_CASE(10) DGOP_GS_CASE(11) DGOP_GS_CASE(12)
+    DGOP_GS_CASE(13) DGOP_GS_CASE(14) DGOP_GS_CASE(15) DGOP_GS_CASE(16)
+#undef DGOP_GS_CASE
+  }
 }
 
 // H(i, j) <- (V_i, w), one block per i, partials summed in the fixed order
@@ -633,11 +693,14 @@ int run_whole(SolverImpl& s, cudaStream_t st, const void* b, const void* x, cons
 
 // After segment `seg` was enqueued: starts the read of its `done` word and reports whether the
 // solve had finished by the end of segment seg - 1 (one segment of look-ahead, whose kernels are
-// no-ops once `done` is set).  Without events the read is synchronous and reports segment seg.
-int segment_done(SolverImpl& s, cudaStream_t st, int seg, bool* stop) {
+// no-ops once `done` is set).  Without events, or without `ahead`, the read is synchronous and
+// reports segment seg.  CG looks ahead (a chunk's no-ops cost less than the host's round trip per
+// chunk); restart cycles do not: the no-op launches of one cycle (30 iterations of 8 kernels, about
+// 0.5 ms) cost more than the round trips (about 15 us each) of the cycles a solve takes.
+int segment_done(SolverImpl& s, cudaStream_t st, int seg, bool* stop, bool ahead = true) {
   int* flag = s.h_flag + (seg & 1);
   DGOP_CUDA_S(cudaMemcpyAsync(flag, s.state, sizeof(int), cudaMemcpyDeviceToHost, st));
-  if (!s.ev[0]) {
+  if (!s.ev[0] || !ahead) {
     DGOP_CUDA_S(cudaStreamSynchronize(st));
     *stop = *flag != 0;
     return DGOP_OK;
@@ -787,7 +850,7 @@ int gmres_solve(SolverImpl& s, const double* b, double* x, int max_iters, double
       for (int c = 0; c <= max_iters; ++c) {
         DGOP_TRY(run_segment(s, st, b, x, cycle));
         bool stop = false;
-        DGOP_TRY(segment_done(s, st, c, &stop));
+        DGOP_TRY(segment_done(s, st, c, &stop, false));
         if (stop) break;
       }
     }
@@ -891,7 +954,7 @@ int gmres_ir_solve(SolverImpl& s, const double* b, double* x, int max_iters, dou
       for (int c = 0; c <= max_iters; ++c) {
         DGOP_TRY(run_segment(s, st, b, x, cycle));
         bool stop = false;
-        DGOP_TRY(segment_done(s, st, c, &stop));
+        DGOP_TRY(segment_done(s, st, c, &stop, false));
         if (stop) break;
       }
     }
