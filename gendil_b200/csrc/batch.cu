@@ -1,11 +1,14 @@
 // Batches of independent operators: one persistent launch per (dimension, order) class.
 //
-// Operators on the any-dimension Kronecker kernel are grouped by (D, N, kernel variant); each
-// group's parameter
-// table (the operators' forward parameters, x and y patched per apply) and the prefix sums of
-// their element batches live on the device, and one launch of kronnd_batch_kernel walks every
+// Operators on the any-dimension Kronecker kernel are grouped by (D, N, kernel variant); each group's
+// parameter table (the operators' forward parameters, x and y patched per apply) and the prefix sums
+// of their element batches live on the device, and one launch of the group's batch kernel walks every
 // element batch of every operator of the group.  Operators on another kernel are applied one
-// launch each.  Results equal those of the operators' own applies bit for bit (same arithmetic).
+// launch each.  The launches are independent, so they are spread over the caller's stream and a
+// few more that fork from it and join it again (largest operators first): a launch's tail, and the
+// small operators, run beside the others (24 systems of 2D to 4D, p = 1..5: 414 us one after another
+// with the grouped kernels, 220 us so and with the split kernels).  Results equal those of the
+// operators' own applies bit for bit (same arithmetic).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -25,9 +28,9 @@ struct BatchGroup {
   std::vector<int> members;                 // indices into the batch
   std::vector<KronNDParams<double>> table;  // host copy (x, y patched per apply)
   std::vector<int64_t> first;
-  KronNDParams<double>* d_table = nullptr;
+  KronNDParams<double>* d_table = nullptr;  // part of the batch's table
   int64_t* d_first = nullptr;
-  KronNDParams<double>* h_pinned = nullptr;  // staging of the table upload
+  KronNDParams<double>* h_pinned = nullptr;  // part of the staging of the table's upload
   int eb = 1;
   size_t smem = 0;
   dim3 grid, block;
@@ -39,6 +42,14 @@ struct dgop_batch {
   std::vector<BatchGroup> groups;
   std::vector<int> singles;  // operators applied one launch each
   cudaEvent_t uploaded = nullptr;
+  // every group's parameter table, uploaded by one copy
+  KronNDParams<double>* d_tables = nullptr;
+  KronNDParams<double>* h_tables = nullptr;
+  size_t table_bytes = 0;
+  // side streams of an apply, their fork and join events
+  std::vector<cudaStream_t> side;
+  std::vector<cudaEvent_t> joined;
+  cudaEvent_t forked = nullptr;
 };
 
 namespace {
@@ -51,10 +62,13 @@ namespace {
 
 void release(dgop_batch* b) {
   for (auto& g : b->groups) {
-    if (g.d_table) cudaFree(g.d_table);
     if (g.d_first) cudaFree(g.d_first);
-    if (g.h_pinned) cudaFreeHost(g.h_pinned);
   }
+  if (b->d_tables) cudaFree(b->d_tables);
+  if (b->h_tables) cudaFreeHost(b->h_tables);
+  for (cudaStream_t s : b->side) cudaStreamDestroy(s);
+  for (cudaEvent_t e : b->joined) cudaEventDestroy(e);
+  if (b->forked) cudaEventDestroy(b->forked);
   if (b->uploaded) cudaEventDestroy(b->uploaded);
 }
 
@@ -81,7 +95,7 @@ int setup(dgop_batch* b) {
       DGOP_CUDA_B(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        max_smem - (int)fa.sharedSizeBytes));
       int per_sm = 0;
-      DGOP_CUDA_B(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, (int)op->n64.block.x,
+      DGOP_CUDA_B(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, op->n64.var[v].threads,
                                                                 op->n64.var[v].smem));
       pit = per_sm_of.emplace(fn, per_sm < 1 ? 1 : per_sm).first;
     }
@@ -102,9 +116,10 @@ int setup(dgop_batch* b) {
       b->groups.back().variant = v;
       b->groups.back().eb = op->n64.var[v].eb;
       b->groups.back().smem = op->n64.var[v].smem;
-      b->groups.back().block = op->n64.block;
+      b->groups.back().block = dim3(op->n64.var[v].threads);
     }
-    b->groups[it->second].members.push_back(i);
+    BatchGroup& group = b->groups[it->second];
+    group.members.push_back(i);
   }
   for (auto& g : b->groups) {
     g.first.push_back(0);
@@ -121,15 +136,37 @@ int setup(dgop_batch* b) {
       g.table.push_back(p);
       g.first.push_back(g.first.back() + (op->sp.nelem + g.eb - 1) / g.eb);
     }
-    const size_t tb = sizeof(KronNDParams<double>) * g.table.size();
-    DGOP_CUDA_B(cudaMalloc(&g.d_table, tb));
-    DGOP_CUDA_B(cudaMallocHost(&g.h_pinned, tb));
+    b->table_bytes += sizeof(KronNDParams<double>) * g.table.size();
     DGOP_CUDA_B(cudaMalloc(&g.d_first, sizeof(int64_t) * g.first.size()));
     DGOP_CUDA_B(cudaMemcpy(g.d_first, g.first.data(), sizeof(int64_t) * g.first.size(), cudaMemcpyHostToDevice));
     const int per_sm = per_sm_of[g.entry->func_batch[g.variant]];
     g.grid = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(g.first.back(), (int64_t)sms * per_sm)));
   }
+  if (b->table_bytes) {
+    DGOP_CUDA_B(cudaMalloc(&b->d_tables, b->table_bytes));
+    DGOP_CUDA_B(cudaMallocHost(&b->h_tables, b->table_bytes));
+    size_t at = 0;
+    for (auto& g : b->groups) {
+      g.d_table = b->d_tables + at;
+      g.h_pinned = b->h_tables + at;
+      at += g.table.size();
+    }
+  }
   DGOP_CUDA_B(cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming));
+  // one launch per group and single operator: as many streams as launches, at most kStreams
+  constexpr size_t kStreams = 6;
+  std::stable_sort(b->singles.begin(), b->singles.end(),
+                   [&](int i, int j) { return b->ops[i]->sp.ndofs > b->ops[j]->sp.ndofs; });
+  const size_t launches = b->groups.size() + b->singles.size();
+  for (size_t k = 1; k < std::min(launches, kStreams); ++k) {
+    cudaStream_t s = nullptr;
+    DGOP_CUDA_B(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    b->side.push_back(s);
+    cudaEvent_t e = nullptr;
+    DGOP_CUDA_B(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    b->joined.push_back(e);
+  }
+  DGOP_CUDA_B(cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming));
   return DGOP_OK;
 }
 
@@ -174,31 +211,53 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     return DGOP_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  // the staging buffers of the previous apply may still be in flight
-  DGOP_CUDA_B(cudaEventSynchronize(b->uploaded));
-  for (auto& g : b->groups) {
-    for (size_t k = 0; k < g.members.size(); ++k) {
-      const int i = g.members[k];
+  for (auto& g : b->groups)
+    for (int i : g.members)
       if (!x[i] || !y[i] || x[i] == y[i]) {
         set_error("dgop_batch_apply: null or aliasing vectors");
         return DGOP_ERR_ARG;
       }
-      g.h_pinned[k] = g.table[k];
-      g.h_pinned[k].x = x[i];
-      g.h_pinned[k].y = y[i];
-    }
-    DGOP_CUDA_B(cudaMemcpyAsync(g.d_table, g.h_pinned, sizeof(KronNDParams<double>) * g.members.size(),
-                                cudaMemcpyHostToDevice, st));
-    g.entry->launch_batch[g.variant](g.d_table, g.d_first, (int)g.members.size(), g.eb, g.grid, g.block, g.smem,
-                                     st);
-    DGOP_CUDA_B(cudaGetLastError());
+  if (!b->groups.empty()) {
+    // the staging buffer of the previous apply may still be in flight
+    DGOP_CUDA_B(cudaEventSynchronize(b->uploaded));
+    for (auto& g : b->groups)
+      for (size_t k = 0; k < g.members.size(); ++k) {
+        const int i = g.members[k];
+        g.h_pinned[k] = g.table[k];
+        g.h_pinned[k].x = x[i];
+        g.h_pinned[k].y = y[i];
+      }
+    DGOP_CUDA_B(cudaMemcpyAsync(b->d_tables, b->h_tables, b->table_bytes, cudaMemcpyHostToDevice, st));
+    DGOP_CUDA_B(cudaEventRecord(b->uploaded, st));
   }
-  DGOP_CUDA_B(cudaEventRecord(b->uploaded, st));
+  // fork: launch k goes to stream k modulo the stream count (0: the caller's)
+  const size_t ns = b->side.size();
+  if (ns) DGOP_CUDA_B(cudaEventRecord(b->forked, st));
+  for (size_t k = 0; k < ns; ++k) DGOP_CUDA_B(cudaStreamWaitEvent(b->side[k], b->forked, 0));
+  size_t next = 0;
+  auto stream_of = [&]() {
+    const size_t k = next++ % (ns + 1);
+    return k == 0 ? st : b->side[k - 1];
+  };
+  int rc = DGOP_OK;
+  // single operators first: the largest are among them
   for (int i : b->singles) {
-    const int rc = dgop_apply(b->ops[i], x[i], y[i], stream);
-    if (rc != DGOP_OK) return rc;
+    rc = dgop_apply(b->ops[i], x[i], y[i], stream_of());
+    if (rc != DGOP_OK) break;
   }
-  return DGOP_OK;
+  for (auto& g : b->groups) {
+    if (rc != DGOP_OK) break;
+    g.entry->launch_batch[g.variant](g.d_table, g.d_first, (int)g.members.size(), g.eb, g.grid, g.block, g.smem,
+                                     stream_of());
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) rc = cuda_fail(e, "batch kernel launch");
+  }
+  // join, also after an error: the caller's stream waits for everything queued
+  for (size_t k = 0; k < ns; ++k) {
+    DGOP_CUDA_B(cudaEventRecord(b->joined[k], b->side[k]));
+    DGOP_CUDA_B(cudaStreamWaitEvent(st, b->joined[k], 0));
+  }
+  return rc;
 }
 
 int dgop_batch_destroy(dgop_batch* b) {
