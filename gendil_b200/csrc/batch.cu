@@ -121,6 +121,15 @@ int setup(dgop_batch* b) {
     BatchGroup& group = b->groups[it->second];
     group.members.push_back(i);
   }
+  // a lone operator of the split variant keeps its own launch, which prefetches its elements
+  for (size_t k = 0; k < b->groups.size();) {
+    if (b->groups[k].variant == 5 && b->groups[k].members.size() == 1) {
+      b->singles.push_back(b->groups[k].members[0]);
+      b->groups.erase(b->groups.begin() + (long)k);
+    } else {
+      ++k;
+    }
+  }
   for (auto& g : b->groups) {
     g.first.push_back(0);
     for (int i : g.members) {

@@ -990,7 +990,7 @@ int setup_kronnd(dgop_operator* op, KronNDCfg<Real>& K, const KronPlanHost& plan
   // thread about one block, within ~110 KB of shared memory (two CTAs per SM)
   const bool paired = pairs_share_factors(plan, s);
   // the mass-only variant (4): operators without advection terms, its own smaller layout
-  for (int v = 1; v < kKronNDVariants; ++v) {
+  for (int v = 1; v < 5; ++v) {
     const bool mass_only = v == 4;
     const int G = mass_only ? entry->mass_g : (v == 3 ? 2 : v + 1);  // paired blocks span two axes
     const void* fn = mass_only ? entry->func_m : entry->func_g[v - 1];
@@ -1023,6 +1023,35 @@ int setup_kronnd(dgop_operator* op, KronNDCfg<Real>& K, const KronPlanHost& plan
     if (per_sm_v < 1) continue;
     const int64_t cv = std::min<int64_t>((s.nelem + ebv - 1) / ebv, (int64_t)device_sm_count(op->device) * per_sm_v);
     K.var[v] = {true, ebv, dim3((unsigned)std::max<int64_t>(cv, 1)), pv * ebv + extra, 0.0f, threads};
+  }
+  // the split variant (5): operators with advection terms
+  if (entry->func_s && plan.has_adv) {
+    const int matp = entry->split_matp, mat = N * N;
+    std::vector<double> padded(plan.mats.size() / mat * matp, 0.0);
+    for (size_t m = 0; m < plan.mats.size() / mat; ++m)
+      std::copy_n(plan.mats.begin() + m * mat, mat, padded.begin() + m * matp);
+    rc = upload<Real>(&K.d_pmats, padded.data(), padded.size());
+    if (rc) return rc;
+    for (KronNDParams<Real>* q : {&p, &K.params_t}) {
+      q->pmats = K.d_pmats;
+      for (int a = 0; a <= D; ++a)
+        for (int k = 0; k < D; ++k) {
+          const KronMat m = a < D ? q->slot[a][k] : q->mslot[k];
+          q->pidx[a][k] = m.off < 0 ? 0 : (int)(m.off / mat);
+          q->pvar[a][k] = m.off >= 0 && m.stride ? 1 : 0;
+        }
+    }
+    const int warps = kKronSplitThreads / 32;
+    const size_t sm = (size_t)entry->split_cta_bytes + (size_t)warps * entry->split_warp_bytes;
+    if (sm <= (size_t)max_smem) {
+      DGOP_CUDA(cudaFuncSetAttribute(entry->func_s, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+      int per_sm_s = 0;
+      DGOP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_s, entry->func_s, kKronSplitThreads, sm));
+      const int ebs = warps * entry->split_epw;
+      const int64_t cs = std::min<int64_t>((s.nelem + ebs - 1) / ebs, (int64_t)device_sm_count(op->device) * per_sm_s);
+      if (per_sm_s >= 1)
+        K.var[5] = {true, ebs, dim3((unsigned)std::max<int64_t>(cs, 1)), sm, 0.0f, kKronSplitThreads};
+    }
   }
   K.variant = 0;
   if constexpr (sizeof(Real) == 4) {
@@ -1065,6 +1094,7 @@ void launch_kronnd_variant(const KronNDCfg<Real>& K, int v, KronNDParams<Real> p
   p.eb = L.eb;
   if (v == 0) K.entry->launch(p, L.grid, K.block, L.smem, st);
   else if (v == 4) K.entry->launch_m(p, L.grid, dim3(L.threads), L.smem, st);
+  else if (v == 5) K.entry->launch_s(p, L.grid, dim3(L.threads), L.smem, st);
   else K.entry->launch_g[v - 1](p, L.grid, K.block, L.smem, st);
 }
 
@@ -1143,6 +1173,7 @@ template <typename Real>
 void free_kronnd(KronNDCfg<Real>& K) {
   if (K.d_tc_tiles) cudaFree(K.d_tc_tiles);
   if (K.d_tc_scale) cudaFree(K.d_tc_scale);
+  if (K.d_pmats) cudaFree(K.d_pmats);
   if (K.d_mats) cudaFree(K.d_mats);
   if (K.d_phi) cudaFree(K.d_phi);
   if (K.d_sgn) cudaFree(K.d_sgn);

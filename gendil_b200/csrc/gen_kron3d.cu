@@ -22,7 +22,7 @@ const char* const kKronVariantNames[kKronVariants] = {"stage2-tile", "stage1-til
                                                       "tma1-tile",   "tma2-shfl",   "tma2-tile"};
 // (the any-dimension kernel's variants, kronnd_kernel.cuh, named here with the 3D kernel's)
 const char* const kKronNDVariantNames[kKronNDVariants] = {"nd-passes", "nd-grouped2", "nd-grouped3", "nd-paired",
-                                                          "nd-mass"};
+                                                          "nd-mass", "nd-split"};
 #endif
 
 namespace {

@@ -4,6 +4,7 @@
 #include "kronnd_diff_grad_kernel.cuh"
 #include "kronnd_diff_kernel.cuh"
 #include "kronnd_kernel.cuh"
+#include "kronnd_split_kernel.cuh"
 #include "kronnd_tc_kernel.cuh"
 
 #ifndef DGOP_GEN_D
@@ -54,6 +55,17 @@ void launch_kronnd_paired(const KronNDParams<Real>& p, dim3 grid, dim3 block, si
 }
 
 template <int D, int N, typename Real>
+void launch_kronnd_split(const KronNDParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+  kronnd_split_kernel<D, N, Real><<<grid, block, smem, s>>>(p);
+}
+
+template <int D, int N, typename Real>
+void launch_kronnd_split_batch(const KronNDParams<Real>* table, const int64_t* first, int count, int, dim3 grid,
+                               dim3 block, size_t smem, cudaStream_t s) {
+  kronnd_split_batch_kernel<D, N, Real><<<grid, block, smem, s>>>(table, first, count);
+}
+
+template <int D, int N, typename Real>
 void launch_kronnd_diff(const KronDiffParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
   kronnd_diff_kernel<D, N, Real><<<grid, block, smem, s>>>(p);
 }
@@ -99,6 +111,18 @@ void fill(KronNDEntry<Real>& d) {
       if constexpr (sizeof(Real) == 8) {
         d.launch_batch[3] = &launch_kronnd_batch<D, N, 3, Real>;
         d.func_batch[3] = reinterpret_cast<const void*>(&kronnd_batch_kernel<D, N, 3, Real>);
+      }
+    }
+    if constexpr (SplitShape<D, N>::OK) {
+      d.launch_s = &launch_kronnd_split<D, N, Real>;
+      d.func_s = reinterpret_cast<const void*>(&kronnd_split_kernel<D, N, Real>);
+      d.split_cta_bytes = SplitShape<D, N>::template cta_bytes<Real>(split_matp<N, Real>());
+      d.split_warp_bytes = SplitShape<D, N>::template warp_bytes<Real>();
+      d.split_epw = SplitShape<D, N>::EPW;
+      d.split_matp = split_matp<N, Real>();
+      if constexpr (D == 2 && N == 2 && sizeof(Real) == 8) {
+        d.launch_batch[5] = &launch_kronnd_split_batch<D, N, Real>;
+        d.func_batch[5] = reinterpret_cast<const void*>(&kronnd_split_batch_kernel<D, N, Real>);
       }
     }
     if constexpr (sizeof(Real) == 4 && KronTCShape<D, N>::OK && KronTCShape<D, N>::WARP_BYTES * 4 <= 200 * 1024) {

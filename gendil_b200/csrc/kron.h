@@ -143,6 +143,10 @@ struct KronNDParams {
   const Real* elem[kMaxDim];
   const Real* elem_mass;
   const int* skip;
+  // the split variant's copy of the matrix table, every matrix padded to a multiple of 16 bytes:
+  // slot (a, k)'s matrix is number pidx + c_k pvar (a == D: the mass term)
+  const Real* pmats;
+  int pidx[kMaxDim + 1][kMaxDim], pvar[kMaxDim + 1][kMaxDim];
   // tensor-core variant (kronnd_tc_kernel.cuh, FP32 operators): BF16 Kronecker products of every
   // term's tangential matrices over the fast half (h = 0) and the slow half (h = 1) of the axes,
   // padded tiles; the tile of term t, half h for an element with coordinates c is number

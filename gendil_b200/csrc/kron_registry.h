@@ -9,6 +9,7 @@ namespace dgop {
 
 constexpr int kKronThreads = 128;
 constexpr int kKronNDThreads = 256;  // threads per CTA of the any-dimension kernel
+constexpr int kKronSplitThreads = 64;   // split variant: two warps per CTA, each on its own elements
 constexpr int kKronTCThreads = 128;  // tensor-core variant: four warps (elements) per CTA
 
 // Kernel variants of one (N, precision); the autotuner picks one per operator.
@@ -70,8 +71,10 @@ void register_kron3d_n6();
 // autotuner picks one per operator): 0 one shared-memory pass per axis; 1, 2 groups of 2 or 3
 // axes per pass in registers; 3 axes a and a + D/2 paired, the two terms of a pair run together
 // (even D, operators whose term pairs share their other factors); 4 operators without advection
-// terms (mass, mass inverse): groups of 2 axes passed in place, a third of the shared memory.
-constexpr int kKronNDVariants = 5;
+// terms (mass, mass inverse): groups of 2 axes passed in place, a third of the shared memory;
+// 5 operators with advection terms in 2D, 4D and 6D: the axes split into two halves, one shared-memory
+// round trip per term, a warp per 32 / N^(D/2) elements (kronnd_split_kernel.cuh).
+constexpr int kKronNDVariants = 6;
 extern const char* const kKronNDVariantNames[kKronNDVariants];
 
 template <typename Real>
@@ -92,6 +95,11 @@ struct KronNDEntry {
   const void* func_m = nullptr;
   int per_elem_m = 0;
   int mass_g = 2;  // axes per block of the mass-only kernel (3 when N^3 <= 27)
+  // split variant (kronnd_split_kernel.cuh): shared memory per CTA and per warp, elements
+  // per warp, values per matrix
+  void (*launch_s)(const KronNDParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) = nullptr;
+  const void* func_s = nullptr;
+  int split_cta_bytes = 0, split_warp_bytes = 0, split_epw = 0, split_matp = 0;
   // BF16 tensor-core variant (kronnd_tc_kernel.cuh; FP32 parameters, even D, N^(D/2) <= 32)
   void (*launch_tc)(const KronNDParams<float>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) = nullptr;
   const void* func_tc = nullptr;
