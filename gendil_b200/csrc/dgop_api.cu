@@ -1404,10 +1404,13 @@ static int launch_impl(dgop_operator* op, LaunchCfg<Real>& L, KronCfg<Real>& K, 
     set_error("vectors must be aligned to their element size");
     return DGOP_ERR_ARG;
   }
-  // the Kronecker kernel stages element blocks with 16-byte copies; other pointers take the
-  // generic kernel, or are rejected when the operator has none
+  // the 3D register kernel stages element blocks with 16-byte copies; other pointers take the
+  // any-dimension kernel above order 3, else the generic kernel, or are rejected when the operator has
+  // none
   const bool aligned16 = (ax % 16 == 0) && (ay % 16 == 0);
-  if (op->kernel == DGOP_KERNEL_KRON && K.ready && !aligned16 && !L.ready) {
+  const bool nd_unaligned =
+      op->kernel == DGOP_KERNEL_KRON && K.ready && !aligned16 && op->sp.n > 4 && KN.ready;
+  if (op->kernel == DGOP_KERNEL_KRON && K.ready && !aligned16 && !L.ready && !nd_unaligned) {
     set_error("the Kronecker kernel needs 16-byte aligned vectors and the operator has no generic kernel");
     return DGOP_ERR_ARG;
   }
@@ -1474,7 +1477,7 @@ static int launch_impl(dgop_operator* op, LaunchCfg<Real>& L, KronCfg<Real>& K, 
     if (e != cudaSuccess) return cuda_fail(e, "operator kernel launch");
     return DGOP_OK;
   }
-  if (op->kernel == DGOP_KERNEL_KRONND && KN.ready) {
+  if ((op->kernel == DGOP_KERNEL_KRONND && KN.ready) || nd_unaligned) {
     KronNDParams<Real> p = (extra_flags & kTranspose) ? KN.params_t : KN.params;
     p.x = x;
     p.y = y;

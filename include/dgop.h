@@ -154,7 +154,8 @@ int dgop_operator_device_error(const dgop_operator* op, int* error);
 
 /* y = alpha * A x + beta * y (beta == 0: y is not read).  FP64 device pointers, aligned to their
  * element size; the Kronecker-form kernel runs on 16-byte aligned vectors (any cudaMalloc'd or
- * torch-allocated tensor), other alignments take the generic kernel.
+ * torch-allocated tensor), other alignments take the generic kernel (above order 3 the
+ * any-dimension Kronecker kernel).
  * (MassFiniteElementOperator::operator() massoperator.hpp:209, AdvectionOperator::operator()
  * advectionoperator.hpp:1070: both overwrite y.) */
 int dgop_apply(dgop_operator* op, const double* x, double* y, void* stream);

@@ -98,3 +98,20 @@ def test_mass_inverse_stays_limited_to_single_products():
         g.MassInverseOperator(sp, 4, C.Coefficient(constant=1.0, terms=[{0: lambda x: x}]))
     with pytest.raises(g.DGOPError):
         g.MassInverseOperator(g.Space(3, [3, 3, 3], order=2, basis=g.GL), 4, 1.0)
+
+
+@pytest.mark.parametrize("p", [4, 5])
+def test_vectors_off_16_bytes_above_order_3(p):
+    """Vectors aligned to their element size only, and operators without a generic kernel among them,
+    run on the any-dimension kernel above order 3."""
+    sp = g.Space(3, [4, 3, 5], order=p)
+    rng = np.random.default_rng(p)
+    x = torch.from_numpy(rng.uniform(-1, 1, sp.num_dofs)).cuda()
+    off = torch.empty(sp.num_dofs + 1, dtype=torch.float64, device="cuda")
+    out = torch.empty_like(off)
+    off[1:] = x
+    for op in (g.SystemOperator(sp, p + 2, C.velocity_sincos(3), sigma=2.0), g.MassInverseOperator(sp, p + 2, 2.0)):
+        assert op.kernel == "kron", op.kernel_note
+        y = op(x, torch.empty_like(x))
+        for xs, ys in ((off[1:], out[1:]), (x, out[1:]), (off[1:], torch.empty_like(x))):
+            assert rel_max(op(xs, ys).cpu().numpy(), y.cpu().numpy()) <= APPLY_TOL
