@@ -40,7 +40,8 @@ struct dgop_batch {
   std::vector<dgop_operator*> ops;
   std::vector<BatchGroup> groups;
   std::vector<int> singles;  // operators applied one launch each
-  cudaEvent_t uploaded = nullptr;
+  cudaEvent_t uploaded = nullptr;  // the staging buffer has been read
+  cudaEvent_t applied = nullptr;   // the last apply's launches are done with the device tables
   // every group's parameter table, uploaded by one copy
   KronNDParams<double>* d_tables = nullptr;
   KronNDParams<double>* h_tables = nullptr;
@@ -69,6 +70,7 @@ void release(dgop_batch* b) {
   for (cudaEvent_t e : b->joined) cudaEventDestroy(e);
   if (b->forked) cudaEventDestroy(b->forked);
   if (b->uploaded) cudaEventDestroy(b->uploaded);
+  if (b->applied) cudaEventDestroy(b->applied);
 }
 
 int setup(dgop_batch* b) {
@@ -161,6 +163,7 @@ int setup(dgop_batch* b) {
     }
   }
   DGOP_CUDA_B(cudaEventCreateWithFlags(&b->uploaded, cudaEventDisableTiming));
+  DGOP_CUDA_B(cudaEventCreateWithFlags(&b->applied, cudaEventDisableTiming));
   // one launch per group and single operator: as many streams as launches, at most kStreams
   constexpr size_t kStreams = 6;
   std::stable_sort(b->singles.begin(), b->singles.end(),
@@ -235,6 +238,8 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
         g.h_pinned[k].x = x[i];
         g.h_pinned[k].y = y[i];
       }
+    // and its kernels, on whatever stream it ran, may still read the device tables
+    DGOP_CUDA_B(cudaStreamWaitEvent(st, b->applied, 0));
     DGOP_CUDA_B(cudaMemcpyAsync(b->d_tables, b->h_tables, b->table_bytes, cudaMemcpyHostToDevice, st));
     DGOP_CUDA_B(cudaEventRecord(b->uploaded, st));
   }
@@ -265,12 +270,13 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     DGOP_CUDA_B(cudaEventRecord(b->joined[k], b->side[k]));
     DGOP_CUDA_B(cudaStreamWaitEvent(st, b->joined[k], 0));
   }
+  if (!b->groups.empty()) DGOP_CUDA_B(cudaEventRecord(b->applied, st));
   return rc;
 }
 
 int dgop_batch_destroy(dgop_batch* b) {
   if (!b) return DGOP_OK;
-  if (b->uploaded) cudaEventSynchronize(b->uploaded);
+  if (b->applied) cudaEventSynchronize(b->applied);
   release(b);
   delete b;
   return DGOP_OK;

@@ -175,3 +175,37 @@ def test_batch_solver_reports_unconverged_systems():
     xs = [torch.zeros_like(b) for b in bs]
     res, _ = batch.solve(bs, xs, 3, 1e-14)
     assert all(not r["success"] and r["iterations"] == 3 and r["relative_error"] > 1e-14 for r in res)
+
+
+def _passes_ops(count, rng):
+    """`count` operators of one group whose batch kernel runs for hundreds of microseconds (one
+    shared-memory pass per axis, 110,592 DoFs each)."""
+    ops = []
+    for _ in range(count):
+        o = g.SystemOperator(_space(3, 12, 3), 5, C.velocity_constant(list(rng.uniform(-1, 1, 3))), sigma=1e3)
+        o.select_kernel("kronnd")
+        o.set_variant("nd-passes")
+        ops.append(o)
+    return ops
+
+
+def test_batch_on_two_streams_without_a_wait():
+    """Applies of one batch on two unordered streams, different vectors each: the second apply's
+    parameter table must not replace the first one's under its kernels."""
+    rng = np.random.default_rng(3)
+    ops = _passes_ops(24, rng)
+    ops += [g.SystemOperator(_space(2, [9, 7], 3), 5, C.velocity_constant([0.3, -0.4]), sigma=1e3) for _ in range(3)]
+    batch = g.Batch(ops)
+    assert batch.groups >= 1
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    xs = [[torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops] for _ in streams]
+    want = [[o(x, torch.empty_like(x)) for o, x in zip(ops, v)] for v in xs]
+    for _ in range(10):
+        ys = [[torch.full_like(x, float("nan")) for x in v] for v in xs]
+        torch.cuda.synchronize()
+        for s, x, y in zip(streams, xs, ys):
+            batch.apply(x, y, stream=s)
+        torch.cuda.synchronize()
+        for w, y in zip(want, ys):
+            assert all(torch.equal(a, b) for a, b in zip(w, y))
+    batch.close()
