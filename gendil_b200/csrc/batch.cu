@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <map>
+#include <mutex>
 #include <tuple>
 #include <new>
 #include <vector>
@@ -42,6 +43,7 @@ struct dgop_batch {
   std::vector<int> singles;  // operators applied one launch each
   cudaEvent_t uploaded = nullptr;  // the staging buffer has been read
   cudaEvent_t applied = nullptr;   // the last apply's launches are done with the device tables
+  std::mutex mutex;                // an apply's events and staging are one thread's at a time
   // every group's parameter table, uploaded by one copy
   KronNDParams<double>* d_tables = nullptr;
   KronNDParams<double>* h_tables = nullptr;
@@ -222,6 +224,7 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     return DGOP_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
+  std::lock_guard<std::mutex> lock(b->mutex);
   for (auto& g : b->groups)
     for (int i : g.members)
       if (!x[i] || !y[i] || x[i] == y[i]) {

@@ -209,3 +209,34 @@ def test_batch_on_two_streams_without_a_wait():
         for w, y in zip(want, ys):
             assert all(torch.equal(a, b) for a, b in zip(w, y))
     batch.close()
+
+
+def test_batch_applied_by_two_threads():
+    """Two host threads apply one batch, each on a stream of its own."""
+    import threading
+    rng = np.random.default_rng(4)
+    ops = _passes_ops(4, rng) + [g.SystemOperator(_space(3, n, 3), 5, C.velocity_constant([0.5, -0.2, 0.1]), sigma=1e3)
+                                 for n in ([5, 4, 3], [8, 3, 2], [7, 7, 7])]
+    batch = g.Batch(ops)
+    xs = [[torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops] for _ in range(2)]
+    want = [[o(x, torch.empty_like(x)) for o, x in zip(ops, v)] for v in xs]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            for _ in range(20):
+                ys = [torch.full_like(x, float("nan")) for x in xs[k]]
+                batch.apply(xs[k], ys, stream=s)
+                s.synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(want[k], ys)):
+                    wrong.append(k)
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    batch.close()
