@@ -41,6 +41,7 @@ struct dgop_batch {
   std::vector<dgop_operator*> ops;
   std::vector<BatchGroup> groups;
   std::vector<int> singles;  // operators applied one launch each
+  std::vector<size_t> lane;  // stream of every launch, the singles' then the groups' (0: the caller's)
   cudaEvent_t uploaded = nullptr;  // the staging buffer has been read
   cudaEvent_t applied = nullptr;   // the last apply's launches are done with the device tables
   std::mutex mutex;                // an apply's events and staging are one thread's at a time
@@ -180,6 +181,21 @@ int setup(dgop_batch* b) {
     b->joined.push_back(e);
   }
   DGOP_CUDA_B(cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming));
+  // launches in turn over the streams; an operator whose applies write memory of its own keeps one
+  // stream for all its members, which run in the order of the list there
+  std::map<const dgop_operator*, size_t> kept;
+  for (size_t k = 0, next = 0; k < launches; ++k) {
+    size_t lane = next % (b->side.size() + 1);
+    if (k < b->singles.size() && applies_share_memory(b->ops[b->singles[k]])) {
+      const auto it = kept.emplace(b->ops[b->singles[k]], lane);
+      if (!it.second) {
+        b->lane.push_back(it.first->second);
+        continue;
+      }
+    }
+    b->lane.push_back(lane);
+    ++next;
+  }
   return DGOP_OK;
 }
 
@@ -246,34 +262,37 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     DGOP_CUDA_B(cudaMemcpyAsync(b->d_tables, b->h_tables, b->table_bytes, cudaMemcpyHostToDevice, st));
     DGOP_CUDA_B(cudaEventRecord(b->uploaded, st));
   }
-  // fork: launch k goes to stream k modulo the stream count (0: the caller's)
+  // fork the side streams, launch, and join them
   const size_t ns = b->side.size();
-  if (ns) DGOP_CUDA_B(cudaEventRecord(b->forked, st));
-  for (size_t k = 0; k < ns; ++k) DGOP_CUDA_B(cudaStreamWaitEvent(b->side[k], b->forked, 0));
+  int rc = DGOP_OK;
+  auto keep = [&](cudaError_t e, const char* what) {
+    if (e != cudaSuccess && rc == DGOP_OK) rc = cuda_fail(e, what);
+    return e == cudaSuccess;
+  };
+  size_t forked = 0;
+  if (ns && keep(cudaEventRecord(b->forked, st), "batch fork"))
+    while (forked < ns && keep(cudaStreamWaitEvent(b->side[forked], b->forked, 0), "batch fork")) ++forked;
   size_t next = 0;
   auto stream_of = [&]() {
-    const size_t k = next++ % (ns + 1);
+    const size_t k = b->lane[next++];
     return k == 0 ? st : b->side[k - 1];
   };
-  int rc = DGOP_OK;
   // single operators first: the largest are among them
   for (int i : b->singles) {
-    rc = dgop_apply(b->ops[i], x[i], y[i], stream_of());
     if (rc != DGOP_OK) break;
+    rc = dgop_apply(b->ops[i], x[i], y[i], stream_of());
   }
   for (auto& g : b->groups) {
     if (rc != DGOP_OK) break;
     g.entry->launch_batch[g.variant](g.d_table, g.d_first, (int)g.members.size(), g.eb, g.grid, g.block, g.smem,
                                      stream_of());
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) rc = cuda_fail(e, "batch kernel launch");
+    keep(cudaGetLastError(), "batch kernel launch");
   }
-  // join, also after an error: the caller's stream waits for everything queued
-  for (size_t k = 0; k < ns; ++k) {
-    DGOP_CUDA_B(cudaEventRecord(b->joined[k], b->side[k]));
-    DGOP_CUDA_B(cudaStreamWaitEvent(st, b->joined[k], 0));
-  }
-  if (!b->groups.empty()) DGOP_CUDA_B(cudaEventRecord(b->applied, st));
+  // join every forked stream, also after an error: the caller's stream waits for what was queued
+  for (size_t k = 0; k < forked; ++k)
+    if (keep(cudaEventRecord(b->joined[k], b->side[k]), "batch join"))
+      keep(cudaStreamWaitEvent(st, b->joined[k], 0), "batch join");
+  if (!b->groups.empty()) keep(cudaEventRecord(b->applied, st), "batch event");
   return rc;
 }
 

@@ -153,6 +153,15 @@ struct dgop_operator {
 };
 
 namespace dgop {
+// Whether applies of this operator write device memory of its own beside y: the generic kernel's global
+// workspace (elements too large for shared memory), or the face words that a bulk-tensor launch
+// rebuilds from per-element velocity factors.  Such applies must not run at the same time.
+inline bool applies_share_memory(const dgop_operator* op) {
+  return op->f64.d_scratch != nullptr || (op->k64.factors && op->k64.d_tma != nullptr);
+}
+}  // namespace dgop
+
+namespace dgop {
 // Optional epilogue of an FP64 apply: partials[b] = sum over CTA b's outputs of z . y in a fixed
 // order, entries past the grid zeroed up to `count`.  Kernels that provide it set `*fused`; for
 // the others the caller computes the product itself.

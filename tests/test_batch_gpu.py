@@ -240,3 +240,24 @@ def test_batch_applied_by_two_threads():
         t.join()
     assert not wrong
     batch.close()
+
+
+def test_batch_with_a_repeated_operator_that_owns_a_workspace():
+    """Several right-hand sides of one operator in a batch, whose element (729 values, 4^6 points) does
+    not fit in shared memory: the generic kernel then works in one global workspace per operator,
+    which the members' applies must use in turn.  Another operator's launches run beside them."""
+    sp = _space(6, [2, 3, 2, 2, 2, 2], 2, g.GL)
+    rng = np.random.default_rng(6)
+    op = g.SystemOperator(sp, 4, C.velocity_constant(list(rng.uniform(-1, 1, 6))), sigma=1e3)
+    assert op.kernel == "generic"
+    other = g.SystemOperator(_space(3, [5, 4, 3], 3), 5, C.velocity_constant([0.5, -0.2, 0.1]), sigma=1e3)
+    ops = [op, other, op, op, other, op, op, op]
+    batch = g.Batch(ops)
+    xs = [torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops]
+    want = [o(x, torch.empty_like(x)) for o, x in zip(ops, xs)]
+    for _ in range(5):
+        ys = [torch.full_like(x, float("nan")) for x in xs]
+        batch.apply(xs, ys)
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(want, ys))
+    batch.close()
