@@ -396,7 +396,7 @@ int launch_kron(const dgop_operator* op, KronCfg<Real>& K, int v, const KronPara
     if constexpr (sizeof(Real) == 8) {
       KronTmaParams<double> T;
       std::memset(&T, 0, sizeof(T));
-      T.k = p;
+      T.k = kron_block<4, false>(p);
       const int rc = tma_maps_cached(K, T, p.x, p.y, op->sp.nelem);
       if (rc != DGOP_OK) return rc;
       const int tr = (p.flags & kTranspose) ? 1 : 0;

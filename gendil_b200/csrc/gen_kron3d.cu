@@ -47,33 +47,35 @@ constexpr auto kernel_entry() {
 
 template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT>
 void launch_kron3d_masked(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+  const auto b = kron_block<N, false>(p);
   if constexpr (masked_forms<N, STAGES, SHFL>()) {
     const int mi = kron_mask_index(p);
     if (mi == 0) {
-      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryNone>()<<<grid, block, smem, s>>>(p);
+      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryNone>()<<<grid, block, smem, s>>>(b);
       return;
     }
     if (mi == 1) {
-      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVarySheared>()<<<grid, block, smem, s>>>(p);
+      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVarySheared>()<<<grid, block, smem, s>>>(b);
       return;
     }
   }
-  kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryRuntime>()<<<grid, block, smem, s>>>(p);
+  kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryRuntime>()<<<grid, block, smem, s>>>(b);
 }
 
 template <int N, typename Real, int STAGES, bool SHFL>
 void launch_kron3d(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
   const bool sep = p.has_adv && p.has_mass && !p.mass_merged && !p.nextra;
   if (p.general) {
+    const auto b = kron_block<N, true>(p);
     if constexpr (std::is_same<Real, double>::value) {
       if (p.dot_partials) {
-        if (sep) kron3d_kernel<N, Real, true, STAGES, SHFL, true, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
-        else kron3d_kernel<N, Real, false, STAGES, SHFL, true, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
+        if (sep) kron3d_kernel<N, Real, true, STAGES, SHFL, true, kVaryRuntime, true><<<grid, block, smem, s>>>(b);
+        else kron3d_kernel<N, Real, false, STAGES, SHFL, true, kVaryRuntime, true><<<grid, block, smem, s>>>(b);
         return;
       }
     }
-    if (sep) kron3d_kernel<N, Real, true, STAGES, SHFL, false, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
-    else kron3d_kernel<N, Real, false, STAGES, SHFL, false, kVaryRuntime, true><<<grid, block, smem, s>>>(p);
+    if (sep) kron3d_kernel<N, Real, true, STAGES, SHFL, false, kVaryRuntime, true><<<grid, block, smem, s>>>(b);
+    else kron3d_kernel<N, Real, false, STAGES, SHFL, false, kVaryRuntime, true><<<grid, block, smem, s>>>(b);
     return;
   }
   if constexpr (std::is_same<Real, double>::value) {

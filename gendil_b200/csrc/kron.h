@@ -61,8 +61,9 @@ constexpr int kron_vec(int N) {
   return N % (16 / (int)sizeof(Real)) == 0 ? 16 / (int)sizeof(Real) : (sizeof(Real) == 4 && N % 2 == 0 ? 2 : 1);
 }
 
+// Launch parameters of the 3D kernels, but for the matrices.
 template <typename Real>
-struct KronParams {
+struct KronHead {
   int64_t nelem;      // < 2^32 (checked by the planner); the launch processes [e_begin, nelem)
   int64_t e_begin;
   FastDiv fdx, fdy;   // element index -> (x, y, z) coordinates
@@ -79,16 +80,12 @@ struct KronParams {
   const Real* mats;                          // element-dependent matrix tables (device)
   int vary[kNumSlots];                       // slot depends on the element coordinate
   KronMat vm[kNumSlots];                     // table of a varying slot
-  Real cm[kNumSlots][kKronMaxN * kKronMaxN]; // matrix of a constant slot (kernel-parameter space)
   const Real* phi[3];            // phi[a][e_a * 2 + s]
   const signed char* sgn[3][3];  // sgn[a][k][e_k] in {-1, 0, 1} (k != a)
   const Real* elem[3];           // per-element beta_a factor or nullptr
   const Real* elem_mass;         // per-element sigma factor or nullptr
-  // general form (kron3d_kernel.cuh): a basis without nodes on the faces (lf: its values there),
-  // and mass terms extra[t] = matrices along x, y, z (a density that is a sum of products)
+  // general form (kron3d_kernel.cuh): a basis without nodes on the faces, and nextra mass terms
   int general, gl, nextra;
-  Real lf[2][kKronMaxN];
-  KronMat extra[kKronMaxExtra][3];
   const uint32_t* eflags;        // face word per element (kron3d_kernel.cuh); null: built in the kernel
   const int* skip;               // device word; the launch does nothing when it is non-zero
   // optional epilogue: dot_partials[b] = sum over CTA b's outputs of dot_z . y (fixed order),
@@ -97,6 +94,32 @@ struct KronParams {
   double* dot_partials;
   int dot_count;
 };
+
+// The same with the matrices, in blocks of MAXN x MAXN values (rows of N): the host keeps blocks for the
+// largest N, a kernel takes its own (kron_block), with the sums of products in the general form alone.
+// The whole block is written for every launch and read through the constant cache, so its size
+// counts in small applies: at N = 4 in FP64 2.3 KB, against 4.4 KB when sized for N = 6 (advection
+// transposed, 37x26x31: see kron3d_p3_kernel.cuh).
+template <typename Real, int MAXN = kKronMaxN, bool GENERAL = true>
+struct KronParams : KronHead<Real> {
+  Real cm[kNumSlots][MAXN * MAXN];               // matrix of a constant slot (kernel-parameter space)
+  Real lf[2][MAXN];                              // basis values at the two faces
+  KronMat extra[GENERAL ? kKronMaxExtra : 1][3]; // extra[t]: matrices along x, y, z of mass term t
+};
+static_assert(sizeof(KronParams<double, 4, false>) <= 2400, "the block of the N = 4 kernels grew");
+
+template <int N, bool GENERAL, typename Real>
+inline KronParams<Real, N, GENERAL> kron_block(const KronParams<Real>& p) {
+  KronParams<Real, N, GENERAL> r;
+  static_cast<KronHead<Real>&>(r) = p;
+  for (int s = 0; s < kNumSlots; ++s)
+    for (int i = 0; i < N * N; ++i) r.cm[s][i] = p.cm[s][i];
+  for (int f = 0; f < 2; ++f)
+    for (int i = 0; i < N; ++i) r.lf[f][i] = p.lf[f][i];
+  for (int t = 0; t < (GENERAL ? kKronMaxExtra : 1); ++t)
+    for (int k = 0; k < 3; ++k) r.extra[t][k] = p.extra[t][k];
+  return r;
+}
 
 // Which slots have element-dependent matrices: a compile-time mask of the 3D kernels (bit k:
 // slot k varies) or kVaryRuntime (read P.vary).  A kernel compiled for one mask carries one code
@@ -109,14 +132,14 @@ constexpr uint32_t kVaryNone = 0u;
 constexpr uint32_t kVarySheared = (1u << kSlotTXY) | (1u << kSlotTYZ);
 
 template <typename Real>
-inline uint32_t kron_vary_mask(const KronParams<Real>& k) {
+inline uint32_t kron_vary_mask(const KronHead<Real>& k) {
   uint32_t m = 0;
   for (int i = 0; i < kNumSlots; ++i)
     if (k.vary[i]) m |= 1u << i;
   return m;
 }
 template <typename Real>
-inline int kron_mask_index(const KronParams<Real>& k) {
+inline int kron_mask_index(const KronHead<Real>& k) {
   const uint32_t m = kron_vary_mask(k);
   return m == kVaryNone ? 0 : (m == kVarySheared ? 1 : -1);
 }

@@ -223,22 +223,22 @@ struct RegMat {
   __device__ __forceinline__ Real operator()(int i, int j) const { return a[i][j]; }
 };
 
-template <int N, typename Real, int SLOT>
+template <int N, typename Real, int SLOT, typename Block>
 struct ParamMat {
-  const KronParams<Real>& P;
+  const Block& P;
   __device__ __forceinline__ Real operator()(int i, int j) const { return P.cm[SLOT][i * N + j]; }
 };
 
 // Whether slot SLOT's matrix depends on the element: from the slot mask the kernel is compiled
 // for (kron.h), or at run time.
 template <int SLOT, uint32_t VM, typename Real>
-__device__ __forceinline__ bool slot_varies(const KronParams<Real>& P) {
+__device__ __forceinline__ bool slot_varies(const KronHead<Real>& P) {
   if constexpr (VM == kVaryRuntime) return P.vary[SLOT] != 0;
   else return ((VM >> SLOT) & 1u) != 0;
 }
 // Slot SLOT's matrix for element coordinate `coord` along its axis (element-dependent slots).
 template <int SLOT, typename Real>
-__device__ __forceinline__ const Real* slot_matrix(const KronParams<Real>& P, uint32_t coord) {
+__device__ __forceinline__ const Real* slot_matrix(const KronHead<Real>& P, uint32_t coord) {
   return P.mats + P.vm[SLOT].off + (int64_t)coord * P.vm[SLOT].stride;
 }
 
@@ -345,24 +345,24 @@ __device__ __forceinline__ void memory_pass_z(const Real* p, const Real (&X)[N][
 }
 
 // X <- (slot SLOT's matrix) X along the first or second plane index.
-template <int N, typename Real, int SLOT, bool FIRST, uint32_t VM>
-__device__ __forceinline__ void kron_pass(const KronParams<Real>& P, uint32_t coord, Real (&X)[N][N]) {
+template <int N, typename Real, int SLOT, bool FIRST, uint32_t VM, typename Block>
+__device__ __forceinline__ void kron_pass(const Block& P, uint32_t coord, Real (&X)[N][N]) {
   if (slot_varies<SLOT, VM>(P)) {
     memory_pass<N, FIRST>(slot_matrix<SLOT>(P, coord), X);
   } else {
-    lines_inplace<N, FIRST>(ParamMat<N, Real, SLOT>{P}, X);
+    lines_inplace<N, FIRST>(ParamMat<N, Real, SLOT, Block>{P}, X);
   }
 }
 
 // Y <- (slot SLOT's matrix) X along the second plane index, or Y += with ACC (the products
 // accumulate onto Y in one multiply-add chain per value).
-template <int N, typename Real, int SLOT, bool ACC, uint32_t VM>
-__device__ __forceinline__ void kron_pass_z(const KronParams<Real>& P, uint32_t coord, const Real (&X)[N][N],
+template <int N, typename Real, int SLOT, bool ACC, uint32_t VM, typename Block>
+__device__ __forceinline__ void kron_pass_z(const Block& P, uint32_t coord, const Real (&X)[N][N],
                                             Real (&Y)[N][N]) {
   if (slot_varies<SLOT, VM>(P)) {
     memory_pass_z<N, ACC>(slot_matrix<SLOT>(P, coord), X, Y);
   } else {
-    const ParamMat<N, Real, SLOT> A{P};
+    const ParamMat<N, Real, SLOT, Block> A{P};
 #pragma unroll
     for (int k = 0; k < N; ++k)
 #pragma unroll
@@ -376,8 +376,8 @@ __device__ __forceinline__ void kron_pass_z(const KronParams<Real>& P, uint32_t 
 }
 
 // One line: w = (slot SLOT's matrix) v.
-template <int N, typename Real, int SLOT, uint32_t VM>
-__device__ __forceinline__ void kron_line(const KronParams<Real>& P, uint32_t coord, const Real (&v)[N], Real (&w)[N]) {
+template <int N, typename Real, int SLOT, uint32_t VM, typename Block>
+__device__ __forceinline__ void kron_line(const Block& P, uint32_t coord, const Real (&v)[N], Real (&w)[N]) {
   if (slot_varies<SLOT, VM>(P)) {
     const Real* p = slot_matrix<SLOT>(P, coord);
 #pragma unroll
@@ -390,7 +390,7 @@ __device__ __forceinline__ void kron_line(const KronParams<Real>& P, uint32_t co
       w[j] = s;
     }
   } else {
-    const ParamMat<N, Real, SLOT> A{P};
+    const ParamMat<N, Real, SLOT, Block> A{P};
 #pragma unroll
     for (int j = 0; j < N; ++j) {
       Real s = A(j, 0) * v[0];
@@ -491,7 +491,7 @@ __device__ __forceinline__ void exchange_tile(Real* tile, int le, int t, bool sl
 
 // Element coordinates (x fastest).
 template <typename Real>
-__device__ __forceinline__ void kron_coords(const KronParams<Real>& P, uint32_t e, uint32_t (&c)[3]) {
+__device__ __forceinline__ void kron_coords(const KronHead<Real>& P, uint32_t e, uint32_t (&c)[3]) {
   uint32_t q;
   P.fdx.divmod(e, q, c[0]);
   P.fdy.divmod(q, c[2], c[1]);
@@ -508,7 +508,7 @@ struct FaceDecision {
 };
 
 template <typename Real>
-__device__ __forceinline__ FaceDecision face_decide(const KronParams<Real>& P, int a, int s, const uint32_t (&c)[3],
+__device__ __forceinline__ FaceDecision face_decide(const KronHead<Real>& P, int a, int s, const uint32_t (&c)[3],
                                                     int64_t e, Real tsign, Real el_self, Real& phi, Real& coef) {
   FaceDecision f{false, false, false, 0};
   const int64_t n = P.sizes[a];
@@ -547,7 +547,7 @@ __device__ __forceinline__ FaceDecision face_decide(const KronParams<Real>& P, i
 }
 
 template <typename Real>
-__device__ __forceinline__ Real tan_sign(const KronParams<Real>& P, int a, const uint32_t (&c)[3]) {
+__device__ __forceinline__ Real tan_sign(const KronHead<Real>& P, int a, const uint32_t (&c)[3]) {
   Real s = Real(1);
 #pragma unroll
   for (int k = 0; k < 3; ++k)
@@ -562,7 +562,7 @@ enum : uint32_t { kFaceCorner = 1u, kFaceNb = 2u, kFaceG = 4u };
 constexpr int kFaceWrap = 18;
 
 template <typename Real>
-__device__ __forceinline__ uint32_t face_word(const KronParams<Real>& P, int64_t e, const uint32_t (&c)[3]) {
+__device__ __forceinline__ uint32_t face_word(const KronHead<Real>& P, int64_t e, const uint32_t (&c)[3]) {
   uint32_t w = 0;
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
@@ -582,13 +582,13 @@ __device__ __forceinline__ uint32_t face_word(const KronParams<Real>& P, int64_t
 // With per-element velocity factors, whose values (and signs) the caller may change between
 // applies: the word from the factors' current values.
 template <typename Real>
-__device__ __noinline__ uint32_t face_word_now(const KronParams<Real>& P, int64_t e) {
+__device__ __noinline__ uint32_t face_word_now(const KronHead<Real>& P, int64_t e) {
   uint32_t c[3];
   kron_coords(P, (uint32_t)e, c);
   return face_word(P, e, c);
 }
 template <typename Real>
-__device__ __forceinline__ uint32_t load_face_word(const KronParams<Real>& P, int64_t e) {
+__device__ __forceinline__ uint32_t load_face_word(const KronHead<Real>& P, int64_t e) {
   return P.eflags ? __ldg(P.eflags + e) : face_word_now(P, e);
 }
 __device__ __forceinline__ uint32_t face_bits(uint32_t w, int a, int s) { return (w >> (3 * (2 * a + s))) & 7u; }
@@ -598,7 +598,7 @@ __device__ __forceinline__ bool face_wraps(uint32_t w, int a, int s) {
 
 // Element offset to the neighbour across face (a, s).
 template <typename Real>
-__device__ __forceinline__ int64_t face_offset(const KronParams<Real>& P, uint32_t w, int a, int s) {
+__device__ __forceinline__ int64_t face_offset(const KronHead<Real>& P, uint32_t w, int a, int s) {
   const int64_t st = a == 0 ? 1 : (a == 1 ? P.sizes[0] : P.sizes[0] * P.sizes[1]);
   const int64_t d = face_wraps(w, a, s) ? -(P.sizes[a] - 1) * st : st;
   return s ? d : -d;
@@ -606,7 +606,7 @@ __device__ __forceinline__ int64_t face_offset(const KronParams<Real>& P, uint32
 // Coefficient of the neighbour's trace on face (a, s): the element's own phi (forward) or, transposed,
 // the neighbour's at its opposite face, times the per-element factor.
 template <typename Real>
-__device__ __forceinline__ Real face_nb_coef(const KronParams<Real>& P, uint32_t w, int a, int s, uint32_t ca, int64_t e,
+__device__ __forceinline__ Real face_nb_coef(const KronHead<Real>& P, uint32_t w, int a, int s, uint32_t ca, int64_t e,
                                              Real k_own) {
   if (!(P.flags & kTranspose)) return k_own;
   const uint32_t cn = face_wraps(w, a, s) ? (s ? 0u : (uint32_t)(P.sizes[a] - 1)) : (s ? ca + 1 : ca - 1);
@@ -632,8 +632,8 @@ __device__ __forceinline__ void trace_row(const Real* p, Real (&v)[N]) {
 // nbrow(s, v): this lane's row of the neighbour's trace on its opposite face.  The trace is the
 // slice there, or with GL (a basis without nodes on the faces) the plane's lines times the basis
 // values P.lf, and a face term goes to every slice with those weights.
-template <int N, typename Real, int A, bool GL, typename Own, typename NbRow>
-__device__ __forceinline__ void plane_faces(const KronParams<Real>& P, uint32_t ca, int64_t e, uint32_t w,
+template <int N, typename Real, int A, bool GL, typename Own, typename NbRow, typename Block>
+__device__ __forceinline__ void plane_faces(const Block& P, uint32_t ca, int64_t e, uint32_t w,
                                             Real (&X)[N][N], Own own, NbRow nbrow) {
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
@@ -684,8 +684,8 @@ __device__ __forceinline__ void plane_faces(const KronParams<Real>& P, uint32_t 
 
 // The z faces' neighbour traces through Tzy: col(s, v) reads column x = t (values y) of the z
 // neighbour's opposite slice, put(s, w) stores the result column in place of it.
-template <int N, typename Real, uint32_t VM, typename Col, typename Put>
-__device__ __forceinline__ void z_faces_prepare(const KronParams<Real>& P, const uint32_t (&c)[3], int64_t e,
+template <int N, typename Real, uint32_t VM, typename Col, typename Put, typename Block>
+__device__ __forceinline__ void z_faces_prepare(const Block& P, const uint32_t (&c)[3], int64_t e,
                                                 uint32_t w, Col col, Put put) {
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
@@ -710,8 +710,8 @@ __device__ __forceinline__ void z_faces_prepare(const KronParams<Real>& P, const
 // Z-face terms added to the accumulator in layout Y: the own trace of an outflow face (X: the z
 // term's lines before Dz, already scaled by the element's factor) and row y = t of the prepared
 // neighbour traces (row(s, v)) through Tzx.
-template <int N, typename Real, uint32_t VM, bool GL, typename Row>
-__device__ __forceinline__ void z_faces_add(const KronParams<Real>& P, const uint32_t (&c)[3], uint32_t w,
+template <int N, typename Real, uint32_t VM, bool GL, typename Row, typename Block>
+__device__ __forceinline__ void z_faces_add(const Block& P, const uint32_t (&c)[3], uint32_t w,
                                             const Real (&X)[N][N], Real (&out)[N][N], Row row) {
 #pragma unroll
   for (int s = 0; s < 2; ++s) {
@@ -786,7 +786,7 @@ __device__ __forceinline__ bool x_slot_taken(uint32_t w, int le, int ne) {  // b
 // Stage the DoFs of elements [e0, e0 + ne) into `buf` (padded layout, coalesced) and, for
 // advection, the neighbour traces the faces in word w will read (lane t copies row t of each).
 template <int N, typename Real>
-__device__ __forceinline__ void stage_group(const KronParams<Real>& P, int64_t e0, int ne, Real* buf, int lane,
+__device__ __forceinline__ void stage_group(const KronHead<Real>& P, int64_t e0, int ne, Real* buf, int lane,
                                             int le, int t, uint32_t w, bool traces = true) {
   using S = Kron3DShape<N, Real>;
   const int nchunks = ne * S::NNN / S::CR;
@@ -832,7 +832,7 @@ constexpr int kron_max_warps = 4;  // warps per CTA of kron3d_kernel (128 thread
 //   GEN:     the general form: with P.gl a basis without nodes on the faces (the neighbours' traces
 //            are formed from their whole elements, read from global memory), and P.nextra mass terms
 template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT, uint32_t VM, bool GEN>
-__device__ __forceinline__ void kron3d_body(const KronParams<Real>& P) {
+__device__ __forceinline__ void kron3d_body(const KronParams<Real, N, GEN>& P) {
   using S = Kron3DShape<N, Real>;
   constexpr int NN = S::NN, NNN = S::NNN, EPW = S::EPW;
   constexpr bool BFLY = SHFL && S::BUTTERFLY;
@@ -1118,14 +1118,14 @@ constexpr int kron3d_min_ctas() {
 template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime,
           bool GEN = false>
 __global__ void __launch_bounds__(128, kron3d_min_ctas<N, Real>())
-    kron3d_kernel(const __grid_constant__ KronParams<Real> P) {
+    kron3d_kernel(const __grid_constant__ KronParams<Real, N, GEN> P) {
   kron3d_body<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>(P);
 }
 
 // Face words of every element (P.eflags of later launches), for operators with advection terms:
 // words[e] of the forward operator, words[nelem + e] of the transposed one.
 template <typename Real>
-__global__ void kron_face_words(const KronParams<Real> fwd, const KronParams<Real> tr, uint32_t* words) {
+__global__ void kron_face_words(const KronHead<Real> fwd, const KronHead<Real> tr, uint32_t* words) {
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < fwd.nelem;
        e += (int64_t)gridDim.x * blockDim.x) {
     uint32_t c[3];

@@ -49,8 +49,8 @@ enum TraceSrc { kTraceLocal = 0, kTraceSlot = 1, kTraceGlobal = 2 };
 // Apply slot SLOT's matrix (for element coordinate `coord` along its axis) along the first or
 // second plane index: constant matrices come from kernel-parameter space.  VM: the slot mask the
 // kernel is compiled for (kron.h).
-template <int N, typename Real, int SLOT, bool FIRST, uint32_t VM = kVaryRuntime>
-__device__ __forceinline__ void p3_apply(const KronParams<Real>& P, uint32_t coord, const Real (&X)[N][N],
+template <int N, typename Real, int SLOT, bool FIRST, uint32_t VM, typename Block>
+__device__ __forceinline__ void p3_apply(const Block& P, uint32_t coord, const Real (&X)[N][N],
                                            Real (&Y)[N][N]) {
   bool vary;
   if constexpr (VM == kVaryRuntime) vary = P.vary[SLOT] != 0;
@@ -72,7 +72,7 @@ __device__ __forceinline__ void p3_apply(const KronParams<Real>& P, uint32_t coo
     if (FIRST) apply_first<N>(A, X, Y);
     else apply_second<N>(A, X, Y);
   } else {
-    ParamMat<N, Real, SLOT> A{P};
+    ParamMat<N, Real, SLOT, Block> A{P};
     if (FIRST) apply_first<N>(A, X, Y);
     else apply_second<N>(A, X, Y);
   }
@@ -105,7 +105,7 @@ __device__ __forceinline__ bool p3_x_in_group(int s, int le, int ne, uint32_t cx
 // e_nb, v) reads this lane's row of the neighbour trace of that side from the group's staged DoFs
 // (x only), the axis' staged trace slot (V-wide), or global memory.
 template <int N, typename Real, bool FIRST, typename NbRow>
-__device__ __forceinline__ void p3_faces(const KronParams<Real>& P, int a, const uint32_t (&c)[3], int64_t e,
+__device__ __forceinline__ void p3_faces(const KronHead<Real>& P, int a, const uint32_t (&c)[3], int64_t e,
                                            uint32_t flags, const Real* rec, const Real (&U)[N][N], Real (&Pm)[N][N],
                                            NbRow nbrow) {
 #pragma unroll
@@ -147,7 +147,7 @@ __device__ __forceinline__ void p3_faces(const KronParams<Real>& P, int a, const
 // also each element's face record and the neighbour traces its faces will read (lane t copies
 // row t of each trace).
 template <int N, typename Real>
-__device__ __forceinline__ void p3_stage_group(const KronParams<Real>& P, int64_t e0, int ne, Real* buf, int lane,
+__device__ __forceinline__ void p3_stage_group(const KronHead<Real>& P, int64_t e0, int ne, Real* buf, int lane,
                                             int le, int t, bool adv) {
   using S = KronP3Shape<N, Real>;
   const int nchunks = ne * S::NNN / S::CR;
@@ -207,7 +207,7 @@ __device__ __forceinline__ void p3_stage_group(const KronParams<Real>& P, int64_
 }
 
 template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT, uint32_t VM>
-__device__ __forceinline__ void kron3d_p3_body(const KronParams<Real>& P) {
+__device__ __forceinline__ void kron3d_p3_body(const KronParams<Real, N, false>& P) {
   using S = KronP3Shape<N, Real>;
   constexpr int NN = S::NN, NNN = S::NNN, EPW = S::EPW;
   constexpr bool BFLY = SHFL && S::BUTTERFLY;
@@ -474,7 +474,7 @@ __device__ __forceinline__ void kron3d_p3_body(const KronParams<Real>& P) {
 // under that cap as the forms with a separate mass term do.
 template <bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime>
 __global__ void __launch_bounds__(128, (!SEP && (VM != kVaryRuntime || STAGES == 1)) ? 4 : 1)
-    kron3d_p3_kernel(const __grid_constant__ KronParams<double> P) {
+    kron3d_p3_kernel(const __grid_constant__ KronParams<double, 4, false> P) {
   kron3d_p3_body<4, double, SEP, STAGES, SHFL, DOT, VM>(P);
 }
 

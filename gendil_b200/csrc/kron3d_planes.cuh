@@ -75,7 +75,7 @@ __device__ __forceinline__ void exchange_tile_dir(Real* tile, int le, int t, boo
 }
 
 template <typename Real>
-__device__ __forceinline__ int64_t neighbour_offset(const KronParams<Real>& P, int a, int s, uint32_t ca) {
+__device__ __forceinline__ int64_t neighbour_offset(const KronHead<Real>& P, int a, int s, uint32_t ca) {
   const int64_t n = P.sizes[a];
   const int64_t st = a == 0 ? 1 : (a == 1 ? P.sizes[0] : P.sizes[0] * P.sizes[1]);
   if (s == 0) return ca > 0 ? -st : (n - 1) * st;

@@ -192,7 +192,7 @@ __device__ __forceinline__ void pass_acc(const Mat& A, const double (&X)[4][4], 
 template <uint32_t VM, int SLOT, bool FIRST, bool ACC>
 __device__ __forceinline__ void tma_apply(const KronTmaParams<double>& T, uint32_t coord, const double* mats,
                                           const double (&X)[4][4], double (&Y)[4][4]) {
-  const KronParams<double>& P = T.k;
+  const auto& P = T.k;
   bool vary;
   if constexpr (VM == kVaryRuntime) vary = P.vary[SLOT] != 0;
   else vary = ((VM >> SLOT) & 1u) != 0;
@@ -224,7 +224,7 @@ __device__ __forceinline__ void tma_apply(const KronTmaParams<double>& T, uint32
     else if constexpr (FIRST) apply_first<4>(A, X, Y);
     else apply_second<4>(A, X, Y);
   } else {
-    ParamMat<4, double, SLOT> A{P};
+    ParamMat<4, double, SLOT, KronParams<double, 4, false>> A{P};
     if constexpr (ACC) pass_acc<FIRST>(A, X, Y);
     else if constexpr (FIRST) apply_first<4>(A, X, Y);
     else apply_second<4>(A, X, Y);
@@ -238,12 +238,12 @@ __device__ __forceinline__ void tma_apply(const KronTmaParams<double>& T, uint32
 // row of the neighbour trace.
 // ph holds phi_0(e_a), phi_1(e_a): the caller loads it (one 16-byte load) before the D pass of
 // axis a, so the pass covers the load's latency.
-__device__ __forceinline__ double2 tma_phi(const KronParams<double>& P, int a, const uint32_t (&c)[3]) {
+__device__ __forceinline__ double2 tma_phi(const KronHead<double>& P, int a, const uint32_t (&c)[3]) {
   return __ldg(reinterpret_cast<const double2*>(P.phi[a] + c[a] * 2));
 }
 
 template <bool FIRST, typename NbRow>
-__device__ __forceinline__ void tma_faces(const KronParams<double>& P, int a, const uint32_t (&c)[3], int64_t e,
+__device__ __forceinline__ void tma_faces(const KronHead<double>& P, int a, const uint32_t (&c)[3], int64_t e,
                                           uint32_t ef, double el, double2 ph, const double (&U)[4][4],
                                           double (&Pm)[4][4], NbRow nbrow) {
 #pragma unroll
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32, 16 / kTmaWarps)
   constexpr int N = 4, EPW = 8;
   using S = Kron3DShape<N, double>;
   static_assert(S::EPW == EPW, "eight elements per warp");
-  const KronParams<double>& P = T.k;
+  const auto& P = T.k;
   // one stage with the exchange tile: the tile is idle from the end of a group until the x faces
   // of the next have been read, so the x-slot element is staged there
   constexpr bool XSLOT = STAGES == 1 && !SHFL;
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32, 16 / kTmaWarps)
 // take one element each and decide its faces exactly as kron3d_kernel does per group
 // (face_decide); the group stages, per axis y and z, the side its elements need most often.
 template <typename Real>
-__global__ void kron_tma_words(const KronParams<Real> P, uint32_t* eflags, uint32_t* gwords) {
+__global__ void kron_tma_words(const KronHead<Real> P, uint32_t* eflags, uint32_t* gwords) {
   const int lane = threadIdx.x & 31;
   const int64_t grp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t e = grp * 8 + lane;

@@ -25,7 +25,7 @@ struct KronTmaParams {
   CUtensorMap ysl;   // x as (4 x, 4 y, 4 z, elements): box 4 x 1 x 4 x 8
   CUtensorMap xel;   // x as rows of 16 values: box 16 x 4 (one element), no swizzle
   CUtensorMap out;   // y as rows of 16 values: box 16 x 32, 128 B swizzle
-  KronParams<Real> k;
+  KronParams<Real, 4, false> k;
   const uint32_t* eflags;  // face word per element
   const uint32_t* gwords;  // slot word per group of 8 elements (group = element / 8)
   int* err;                // set when a bounded wait gives up
