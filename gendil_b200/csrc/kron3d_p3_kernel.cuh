@@ -471,9 +471,11 @@ __device__ __forceinline__ void kron3d_p3_body(const KronParams<Real, N, false>&
 
 // The forms without a separate mass term are held to 128 registers, four CTAs per SM (left to itself
 // the compiler takes 138 for kVarySheared), but for the double-buffered runtime-mask one, which spills
-// under that cap as the forms with a separate mass term do.
+// under that cap as the forms with a separate mass term do.  Those are left to the compiler (no
+// minimum: 134 to 168 registers, three CTAs per SM); a stated minimum of one CTA makes it take up to 192,
+// two per SM (system with a density that varies along x, 36x37x35: 33.4 us, without it 28.3).
 template <bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime>
-__global__ void __launch_bounds__(128, (!SEP && (VM != kVaryRuntime || STAGES == 1)) ? 4 : 1)
+__global__ void __launch_bounds__(128, (!SEP && (VM != kVaryRuntime || STAGES == 1)) ? 4 : 0)
     kron3d_p3_kernel(const __grid_constant__ KronParams<double, 4, false> P) {
   kron3d_p3_body<4, double, SEP, STAGES, SHFL, DOT, VM>(P);
 }
