@@ -652,7 +652,7 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
 }
 
 // Autotuner decisions, shared by the operators of one kernel shape: (kernel family, dimension, N,
-// quadrature, precision, term structure, usable variants, element count within a factor 8).  The first operator of a shape is
+// quadrature, precision, term structure and form, usable variants, element count within a factor 8).  The first operator of a shape is
 // timed; later ones take its variant (dgop_operator_set_variant(-1) times again and replaces it).
 struct TuneKey {
   int family, D, N, Q, precision, structure, usable, size_class;
@@ -670,13 +670,13 @@ std::map<TuneKey, TuneRecord> g_tune_cache;
 thread_local bool g_tune_force = false;  // set by dgop_operator_set_variant(-1)
 
 template <typename Real>
-TuneKey tune_key(const dgop_operator* op, int family, int usable, int has_adv, int has_mass, int merged) {
+TuneKey tune_key(const dgop_operator* op, int family, int usable, int has_adv, int has_mass, int merged, int form = 0) {
   // element counts in classes of a factor 8 (launch shapes and tails change with the size)
   int size_class = 0;
   for (int64_t e = op->sp.nelem; e >= 8; e /= 8) ++size_class;
   return TuneKey{family, op->sp.D, op->sp.n, op->q, (int)sizeof(Real),
                  (op->flags & (kAdvCell | kFaceInt | kFaceBnd | kInvMass | kMass)) | (has_adv << 8) |
-                     (has_mass << 9) | (merged << 10),
+                     (has_mass << 9) | (merged << 10) | (form << 11),
                  usable, size_class};
 }
 
@@ -693,7 +693,13 @@ int autotune_kron(dgop_operator* op, KronCfg<Real>& K) {
     mask |= K.launch[v].ok ? 1 << v : 0;
   }
   if (!K.ready || usable < 2 || op->sp.ndofs > kTuneMaxDofs) return DGOP_OK;
-  const TuneKey key = tune_key<Real>(op, 0, mask, K.params.has_adv, K.params.has_mass, K.params.mass_merged);
+  // the kernels of the 3D family differ by form: the general one (a basis without nodes on the faces,
+  // mass terms of a sum), the slot mask it is compiled for, and per-element velocity factors, for
+  // which a bulk-tensor launch rebuilds its words first
+  const KronParams<Real>& P = K.params;
+  const int form = (P.general != 0) | (P.gl != 0) << 1 | (K.factors ? 1 : 0) << 2 | (kron_mask_index(P) + 1) << 3 |
+                   std::min(P.nextra, 15) << 5;
+  const TuneKey key = tune_key<Real>(op, 0, mask, P.has_adv, P.has_mass, P.mass_merged, form);
   if (!g_tune_force) {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     auto it = g_tune_cache.find(key);

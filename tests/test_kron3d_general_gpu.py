@@ -1,6 +1,8 @@
 """GPU: the 3D register kernel over the orders and forms it takes (p = 0..5, bases without nodes on
 the faces, densities that are sums of products, per-element factors), against the oracle or the
 generic kernel."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -115,3 +117,20 @@ def test_vectors_off_16_bytes_above_order_3(p):
         y = op(x, torch.empty_like(x))
         for xs, ys in ((off[1:], out[1:]), (x, out[1:]), (off[1:], torch.empty_like(x))):
             assert rel_max(op(xs, ys).cpu().numpy(), y.cpu().numpy()) <= APPLY_TOL
+
+
+def test_each_form_is_tuned_on_its_own():
+    """Operators that differ by the kernel they run (basis, per-element factors, which matrices vary), but not
+    in order, quadrature, flags and size, get their own timings whatever was created before them."""
+    sizes = [9, 7, 5]
+    factor = torch.full((math.prod(sizes),), 0.5, dtype=torch.float64, device="cuda")
+    beta = C.velocity_constant([0.7, -0.4, 0.25])
+    ops = [g.AdvectionOperator(g.Space(3, sizes, order=3), 4, beta),
+           g.AdvectionOperator(g.Space(3, sizes, order=3, basis=g.GL), 4, beta),
+           g.AdvectionOperator(g.Space(3, sizes, order=3), 4, C.velocity_bubble(3)),
+           g.AdvectionOperator(g.Space(3, sizes, order=3), 4,
+                               [C.Coefficient(constant=c.constant, element_factor=factor) for c in beta])]
+    times = [tuple(sorted(op.variant_times().items())) for op in ops]
+    assert all(op.kernel == "kron" for op in ops) and len(set(times)) == len(ops)
+    again = g.AdvectionOperator(g.Space(3, sizes, order=3), 4, beta)  # the same form: the record of the first
+    assert tuple(sorted(again.variant_times().items())) == times[0]
