@@ -608,7 +608,9 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     const int threads = kv.threads, warps = threads / 32;
     L.block = dim3(threads);
     L.smem = kv.launch_tma ? (size_t)kv.warp_smem
-                           : (size_t)warps * (p.general ? kv.warp_smem_general : kv.warp_smem) * sizeof(Real);
+                           : (size_t)warps * sizeof(Real) * (p.general                              ? kv.warp_smem_general
+                                                           : K.factors && kron_early_factors(N) ? kv.warp_smem_fact
+                                                                                                : kv.warp_smem);
     if ((int)L.smem > max_smem - 1024) continue;  // 1 KB covers every variant's static shared memory
     int arc = allow_dynamic_smem(kv.func, max_smem);
     if (arc == DGOP_OK) arc = allow_dynamic_smem(kv.func_sep, max_smem);
@@ -621,6 +623,10 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
       for (const auto& by_sep : by_dot)
         for (const void* f : by_sep)
           if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
+    for (const auto& by_dot : kv.func_fact)
+      for (const auto& by_sep : by_dot)
+        for (const void* f : by_sep)
+          if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
     if (arc != DGOP_OK) return arc;
     // resident CTAs per SM of the kernels this operator launches (the slot-mask form when its
     // mask has one), plain and with the inner-product epilogue: each gets a grid of that many
@@ -628,6 +634,8 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     const void* kern[2] = {sep ? kv.func_sep : kv.func, kv.func_dot[sep ? 1 : 0]};
     for (int dot = 0; dot < 2; ++dot)
       if (p.general) kern[dot] = kv.func_general[dot][sep ? 1 : 0];
+      else if (K.factors && kv.func_fact[dot][sep ? 1 : 0][mi + 1]) kern[dot] = kv.func_fact[dot][sep ? 1 : 0][mi + 1];
+      else if (K.factors && kv.func_fact[dot][sep ? 1 : 0][0]) kern[dot] = kv.func_fact[dot][sep ? 1 : 0][0];
       else if (mi >= 0 && kv.func_masked[mi][dot][sep ? 1 : 0]) kern[dot] = kv.func_masked[mi][dot][sep ? 1 : 0];
     int per_sm = 0, per_sm_dot = 0;
     DGOP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[0], threads, L.smem));

@@ -34,32 +34,44 @@ constexpr bool masked_forms() {
   return N >= 4 && STAGES == 1 && !SHFL;
 }
 
-// The kernel of a variant: FP64 N = 4 has its own schedule (kron3d_p3_kernel.cuh).
+// The kernel of a variant: FP64 N = 4 has its own schedule (kron3d_p3_kernel.cuh), and so have (FACT)
+// operators with per-element velocity factors.
 template <int N, typename Real>
 constexpr bool own_schedule() {
   return N == 4 && std::is_same<Real, double>::value;
 }
-template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false>
+template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false, bool FACT = false>
 constexpr auto kernel_entry() {
-  if constexpr (own_schedule<N, Real>() && !GEN) return &kron3d_p3_kernel<SEP, STAGES, SHFL, DOT, VM>;
+  if constexpr ((own_schedule<N, Real>() && !GEN) || FACT) return &kron3d_p3_kernel<N, Real, SEP, STAGES, SHFL, DOT, VM>;
   else return &kron3d_kernel<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>;
 }
 
-template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT>
-void launch_kron3d_masked(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT, bool FACT>
+void launch_kron3d_block(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
   const auto b = kron_block<N, false>(p);
   if constexpr (masked_forms<N, STAGES, SHFL>()) {
     const int mi = kron_mask_index(p);
     if (mi == 0) {
-      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryNone>()<<<grid, block, smem, s>>>(b);
+      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryNone, false, FACT>()<<<grid, block, smem, s>>>(b);
       return;
     }
     if (mi == 1) {
-      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVarySheared>()<<<grid, block, smem, s>>>(b);
+      kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVarySheared, false, FACT>()<<<grid, block, smem, s>>>(b);
       return;
     }
   }
-  kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryRuntime>()<<<grid, block, smem, s>>>(b);
+  kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, kVaryRuntime, false, FACT>()<<<grid, block, smem, s>>>(b);
+}
+// (an operator with advection terms and no face words has per-element velocity factors)
+template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT>
+void launch_kron3d_masked(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem, cudaStream_t s) {
+  if constexpr (kron_early_factors(N)) {
+    if (p.has_adv && !p.eflags) {
+      launch_kron3d_block<N, Real, SEP, STAGES, SHFL, DOT, true>(p, grid, block, smem, s);
+      return;
+    }
+  }
+  launch_kron3d_block<N, Real, SEP, STAGES, SHFL, DOT, false>(p, grid, block, smem, s);
 }
 
 template <int N, typename Real, int STAGES, bool SHFL>
@@ -89,9 +101,19 @@ void launch_kron3d(const KronParams<Real>& p, dim3 grid, dim3 block, size_t smem
   else launch_kron3d_masked<N, Real, false, STAGES, SHFL, false>(p, grid, block, smem, s);
 }
 
-template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false>
+template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT, uint32_t VM, bool GEN = false, bool FACT = false>
 const void* kernel_of() {
-  return reinterpret_cast<const void*>(kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, VM, GEN>());
+  return reinterpret_cast<const void*>(kernel_entry<N, Real, STAGES, SHFL, SEP, DOT, VM, GEN, FACT>());
+}
+
+// The forms for per-element velocity factors: [inner-product epilogue][separate mass term][mask index + 1].
+template <int N, typename Real, int STAGES, bool SHFL, bool SEP, bool DOT>
+void fill_fact(KronVariant<Real>& v) {
+  v.func_fact[DOT][SEP][0] = kernel_of<N, Real, STAGES, SHFL, SEP, DOT, kVaryRuntime, false, true>();
+  if constexpr (masked_forms<N, STAGES, SHFL>()) {
+    v.func_fact[DOT][SEP][1] = kernel_of<N, Real, STAGES, SHFL, SEP, DOT, kVaryNone, false, true>();
+    v.func_fact[DOT][SEP][2] = kernel_of<N, Real, STAGES, SHFL, SEP, DOT, kVarySheared, false, true>();
+  }
 }
 
 template <int N, typename Real, int STAGES, bool SHFL>
@@ -120,6 +142,15 @@ void fill_variant(KronVariant<Real>& v) {
   if constexpr (std::is_same<Real, double>::value) {
     v.func_general[1][0] = kernel_of<N, Real, STAGES, SHFL, false, true, kVaryRuntime, true>();
     v.func_general[1][1] = kernel_of<N, Real, STAGES, SHFL, true, true, kVaryRuntime, true>();
+  }
+  if constexpr (kron_early_factors(N)) {
+    fill_fact<N, Real, STAGES, SHFL, false, false>(v);
+    fill_fact<N, Real, STAGES, SHFL, true, false>(v);
+    if constexpr (std::is_same<Real, double>::value) {
+      fill_fact<N, Real, STAGES, SHFL, false, true>(v);
+      fill_fact<N, Real, STAGES, SHFL, true, true>(v);
+    }
+    v.warp_smem_fact = KronP3Shape<N, Real>::warp_smem(STAGES, SHFL);
   }
   v.warp_smem_general = Kron3DShape<N, Real>::warp_smem(STAGES, SHFL);
   v.warp_smem = own_schedule<N, Real>() ? KronP3Shape<N, Real>::warp_smem(STAGES, SHFL) : v.warp_smem_general;

@@ -61,6 +61,10 @@ constexpr int kron_vec(int N) {
   return N % (16 / (int)sizeof(Real)) == 0 ? 16 / (int)sizeof(Real) : (sizeof(Real) == 4 && N % 2 == 0 ? 2 : 1);
 }
 
+// Orders at which operators with per-element velocity factors, whose faces are decided in every apply, run
+// the earlier schedule (kron3d_p3_kernel.cuh).
+constexpr bool kron_early_factors(int N) { return N <= 4; }
+
 // Launch parameters of the 3D kernels, but for the matrices.
 template <typename Real>
 struct KronHead {

@@ -1,5 +1,6 @@
-// The 3D register kernel's FP64 form for N = p + 1 = 4, without the general features: same layouts,
-// variants and staging as kron3d_kernel.cuh with another schedule,
+// The 3D register kernel's earlier schedule, without the general features: FP64 operators at N = p + 1 =
+// 4, and for N <= 4 in both precisions operators with per-element velocity factors.  Same layouts,
+// variants and staging as kron3d_kernel.cuh,
 //
 //   Z: px = Dx u + x-faces ; qx = Txy px ; py = Dy u + y-faces             exchange qx, py -> Y
 //   Y: out = Txz qx + Tyx Tyz py ; pz = Dz u + z-faces (mass merged) ; qz = Tzx pz
@@ -11,7 +12,11 @@
 // vectors and 128 registers hold what either schedule keeps, this one is the faster: us per apply
 // here / there 16.2 / 16.5 (37x26x31 sheared advection), 52.9 / 56.6 (47x48x48, every velocity
 // component varying along its own axis), 23.1 / 24.5 (mass, 47x48x48).  In FP32 and at N = 2, 3 the other
-// measured faster (FP32 48^3: 31.0 / 26.5; N = 3, 80^3: 168 / 135).
+// measured faster (FP32 48^3: 31.0 / 26.5; N = 3, 80^3: 168 / 135), but not with velocity factors: their
+// values and signs may change between applies, so that the face words the other schedule reads have to
+// be made in the kernel, ahead of the copies they decide on, where this one's staging decides each face
+// once and keeps its coefficients (implicit system with factors, p = 1, 16x17x15 5.3 / 6.9,
+// transposed 72x73x71 43.7 / 51.9; p = 0, 144x145x143 105.7 / 119.4; FP32 p = 3, 36x37x35 16.3 / 19.0).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -469,15 +474,15 @@ __device__ __forceinline__ void kron3d_p3_body(const KronParams<Real, N, false>&
   }
 }
 
-// The forms without a separate mass term are held to 128 registers, four CTAs per SM (left to itself
+// At N = 4 in FP64 the forms without a separate mass term are held to 128 registers, four CTAs per SM (left to itself
 // the compiler takes 138 for kVarySheared), but for the double-buffered runtime-mask one, which spills
 // under that cap as the forms with a separate mass term do.  Those are left to the compiler (no
 // minimum: 134 to 168 registers, three CTAs per SM); a stated minimum of one CTA makes it take up to 192,
 // two per SM (system with a density that varies along x, 36x37x35: 33.4 us, without it 28.3).
-template <bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime>
-__global__ void __launch_bounds__(128, (!SEP && (VM != kVaryRuntime || STAGES == 1)) ? 4 : 0)
-    kron3d_p3_kernel(const __grid_constant__ KronParams<double, 4, false> P) {
-  kron3d_p3_body<4, double, SEP, STAGES, SHFL, DOT, VM>(P);
+template <int N, typename Real, bool SEP, int STAGES, bool SHFL, bool DOT = false, uint32_t VM = kVaryRuntime>
+__global__ void __launch_bounds__(128, (N == 4 && sizeof(Real) == 8 && !SEP && (VM != kVaryRuntime || STAGES == 1)) ? 4 : 0)
+    kron3d_p3_kernel(const __grid_constant__ KronParams<Real, N, false> P) {
+  kron3d_p3_body<N, Real, SEP, STAGES, SHFL, DOT, VM>(P);
 }
 
 }  // namespace dgop

@@ -37,8 +37,12 @@ struct KronVariant {
   const void* func_masked[2][2][2] = {};
   // the general form (KronParams::general): [with the inner-product epilogue][separate mass term]
   const void* func_general[2][2] = {};
+  // the forms for per-element velocity factors (kron_early_factors): [with the inner-product epilogue]
+  // [separate mass term][0: run-time slot mask, mask index + 1]
+  const void* func_fact[2][2][3] = {};
   int warp_smem = 0;               // Real values of shared memory per warp (bytes per CTA for bulk-tensor variants)
   int warp_smem_general = 0;       // Real values per warp of the general form
+  int warp_smem_fact = 0;          // and of the forms for velocity factors
   int threads = 0;                 // threads per CTA
 };
 
