@@ -1338,7 +1338,8 @@ int create_operator(const dgop_space* space, int q, const dgop_coef* sigma, cons
       op->kron_why = plan.why;
     }
   }
-  if (op->kernel == DGOP_KERNEL_KRONND) {
+  // (above order 3 the register kernel's operators run there too, for vectors off 16 bytes)
+  if (op->kernel == DGOP_KERNEL_KRONND || (op->kernel == DGOP_KERNEL_KRON && op->sp.n > 4)) {
     autotune_kronnd(op, op->n64);
     autotune_kronnd(op, op->n32);
   }

@@ -134,3 +134,15 @@ def test_each_form_is_tuned_on_its_own():
     assert all(op.kernel == "kron" for op in ops) and len(set(times)) == len(ops)
     again = g.AdvectionOperator(g.Space(3, sizes, order=3), 4, beta)  # the same form: the record of the first
     assert tuple(sorted(again.variant_times().items())) == times[0]
+
+
+@pytest.mark.parametrize("p", [4, 5])
+def test_any_dimension_kernel_of_register_operators_is_tuned(p):
+    """Above order 3, where vectors off 16 bytes run on the any-dimension kernel, its variants are timed at
+    creation as for the operators that always run there."""
+    sp = g.Space(3, [6, 5, 4], order=p)
+    for op in (g.SystemOperator(sp, p + 2, C.velocity_sincos(3), sigma=2.0), g.MassOperator(sp, p + 2, 2.0)):
+        assert op.kernel == "kron", op.kernel_note
+        op.select_kernel("kronnd")
+        times = {k: t for k, t in op.variant_times().items() if t > 0.0}
+        assert len(times) >= 2 and times[op.variant] == min(times.values())
