@@ -1310,10 +1310,20 @@ int create_operator(const dgop_space* space, int q, const dgop_coef* sigma, cons
     // any-dimension kernel: every shape the Kronecker form covers (also the 3D register kernel's,
     // where it is an alternative the caller may select)
     KronPlanHost plan_nd = plan_kron(in);
+    // A mass operator on a basis without nodes on the faces takes it where it beats the generic kernel:
+    // with the mass-only variant (2D and up, order <= 5), and in 3D.  Elsewhere one shared-memory
+    // pass per axis is left, and the generic kernel is the faster (us, generic / any-dimension: 1D p = 4,
+    // 600,000 DoFs 36 / 115; 2D p = 5, 289x290 62 / 40; 2D p = 6, 247x248 54 / 71; 3D p = 6, 21x22x20 68 /
+    // 40, in FP32 48 / 30 but 10x11x9 9.2 / 9.8).
+    const bool gl_mass = plan_nd.ok && !in.gll;
+    if (gl_mass && op->f64.ready && !(kronnd_slot_f64(in.D, in.N).func_m || (in.D == 3 && in.N >= 7)))
+      plan_nd.ok = false;
+    const bool nd_f32 =
+        !(gl_mass && op->f32.ready && !kronnd_slot_f32(in.D, in.N).func_m && op->sp.nelem < 4096);
     if (plan_nd.ok && (int64_t)op->sp.nelem < (int64_t(1) << 40)) {
       const double* es = sg ? sg->element_factor : nullptr;
       if (setup_kronnd<double>(op, op->n64, plan_nd, es, elem_beta) == DGOP_OK) {
-        if (setup_kronnd<float>(op, op->n32, plan_nd, es, elem_beta) != DGOP_OK) free_kronnd(op->n32);
+        if (!nd_f32 || setup_kronnd<float>(op, op->n32, plan_nd, es, elem_beta) != DGOP_OK) free_kronnd(op->n32);
         op->kernel = DGOP_KERNEL_KRONND;
       } else {
         free_kronnd(op->n64);

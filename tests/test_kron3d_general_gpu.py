@@ -146,3 +146,17 @@ def test_any_dimension_kernel_of_register_operators_is_tuned(p):
         op.select_kernel("kronnd")
         times = {k: t for k, t in op.variant_times().items() if t > 0.0}
         assert len(times) >= 2 and times[op.variant] == min(times.values())
+
+
+@pytest.mark.parametrize("D,p,kernel", [(1, 1, "generic"), (1, 4, "generic"), (2, 1, "kronnd"), (2, 5, "kronnd"),
+                                        (2, 6, "generic"), (3, 3, "kron"), (3, 6, "kronnd"), (4, 1, "kronnd")])
+def test_gauss_legendre_mass_takes_the_faster_kernel(D, p, kernel):
+    """The any-dimension kernel where it has its mass-only variant, and in 3D; the generic kernel, as for
+    every basis without face nodes, elsewhere.  Same values on either."""
+    sp = g.Space(D, [5, 3, 4, 2][:D], order=p, basis=g.GL)
+    op = g.MassOperator(sp, p + 1, 1.5)
+    assert op.kernel == kernel, op.kernel_note
+    x = np.random.default_rng(D + p).uniform(-1, 1, sp.num_dofs)
+    y, y32 = cuda_apply(op, x), cuda_apply(op, x, f32=True)
+    op.select_kernel("generic")
+    assert rel_max(y, cuda_apply(op, x)) <= APPLY_TOL and rel_max(y32, y) <= 1e-5
