@@ -1337,6 +1337,10 @@ int create_operator(const dgop_space* space, int q, const dgop_coef* sigma, cons
       if (krc == DGOP_OK) {
         if (setup_kron<float>(op, op->k32, plan, es, elem_beta, t.Bf) != DGOP_OK) free_kron(op->k32);
         op->kernel = DGOP_KERNEL_KRON;
+        // FP32 mass operators at p = 4: five floats fit no vector access of the register kernel, while the
+        // mass-only variant of the any-dimension kernel keeps its threads busy (us, register / mass-only:
+        // 29x30x28 13.0 / 9.6, 6x7x5 4.7 / 4.2; at p = 5, 24x25x23, 9.9 / 12.0)
+        op->n32.preferred = op->sp.n == 5 && op->n32.ready && op->n32.var[4].ok && !plan.nextra;
         autotune_kron(op, op->k64);
         autotune_kron(op, op->k32);
       } else {
@@ -1431,11 +1435,11 @@ static int launch_impl(dgop_operator* op, LaunchCfg<Real>& L, KronCfg<Real>& K, 
   }
   // the 3D register kernel stages element blocks with 16-byte copies; other pointers take the
   // any-dimension kernel above order 3, else the generic kernel, or are rejected when the operator has
-  // none
+  // none.  The any-dimension kernel is also preferred where it is the faster (create_operator).
   const bool aligned16 = (ax % 16 == 0) && (ay % 16 == 0);
-  const bool nd_unaligned =
-      op->kernel == DGOP_KERNEL_KRON && K.ready && !aligned16 && op->sp.n > 4 && KN.ready;
-  if (op->kernel == DGOP_KERNEL_KRON && K.ready && !aligned16 && !L.ready && !nd_unaligned) {
+  const bool nd_instead =
+      op->kernel == DGOP_KERNEL_KRON && KN.ready && (KN.preferred || (K.ready && !aligned16 && op->sp.n > 4));
+  if (op->kernel == DGOP_KERNEL_KRON && K.ready && !aligned16 && !L.ready && !nd_instead) {
     set_error("the Kronecker kernel needs 16-byte aligned vectors and the operator has no generic kernel");
     return DGOP_ERR_ARG;
   }
@@ -1502,7 +1506,7 @@ static int launch_impl(dgop_operator* op, LaunchCfg<Real>& L, KronCfg<Real>& K, 
     if (e != cudaSuccess) return cuda_fail(e, "operator kernel launch");
     return DGOP_OK;
   }
-  if ((op->kernel == DGOP_KERNEL_KRONND && KN.ready) || nd_unaligned) {
+  if ((op->kernel == DGOP_KERNEL_KRONND && KN.ready) || nd_instead) {
     KronNDParams<Real> p = (extra_flags & kTranspose) ? KN.params_t : KN.params;
     p.x = x;
     p.y = y;

@@ -95,6 +95,7 @@ struct KronNDCfg {
     int threads = kKronNDThreads;
   } var[kKronNDVariants];
   int variant = 0;
+  bool preferred = false;   // a 3D register-kernel operator's applies run here
   Real* d_pmats = nullptr;  // the split variant's padded matrix table
   // BF16 tensor-core launch (FP32 configuration only) and its Kronecker tile tables
   bool tc_ok = false;
