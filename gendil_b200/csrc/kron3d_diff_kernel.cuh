@@ -551,8 +551,9 @@ __global__ void __launch_bounds__(128, N <= 4 ? 3 : 2)
       double s = 0.0;
       for (int w = 0; w < nw; ++w) s += wsum[w];
       P.dot_partials[blockIdx.x] = s;
-      for (int i = blockIdx.x + gridDim.x; i < P.dot_count; i += gridDim.x) P.dot_partials[i] = 0.0;
     }
+    for (int i = gridDim.x + blockIdx.x * blockDim.x + threadIdx.x; i < P.dot_count; i += gridDim.x * blockDim.x)
+      P.dot_partials[i] = 0.0;
   }
 }
 
