@@ -1466,7 +1466,7 @@ static int launch_impl(dgop_operator* op, LaunchCfg<Real>& L, KronCfg<Real>& K, 
       set_error("the transposed interior-penalty operator is provided for the symmetric form (sigma = -1) only");
       return DGOP_ERR_UNSUPPORTED;
     }
-    if (SD.entry3d && aligned16) {
+    if (SD.apply3d && aligned16) {
       Kron3DDiffParams<Real> p = SD.params3d;  // symmetric for sigma = -1: the transpose is the operator
       p.x = x;
       p.y = y;

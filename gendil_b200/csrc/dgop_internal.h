@@ -116,6 +116,7 @@ struct KronDiffCfg {
   Real* d_mu = nullptr;  // FP32 copy of the per-element diffusivity
   // 3D register kernel (orders 1..5; 16-byte aligned vectors), plain and with the inner-product epilogue
   const KronEntry<Real>* entry3d = nullptr;
+  bool apply3d = false;  // the apply runs on it (the gradient always does)
   Kron3DDiffParams<Real> params3d{};
   bool gll = true;
   dim3 grid3d[3], block3d;  // grids by DiffMode: apply, apply with the epilogue, coefficient gradient

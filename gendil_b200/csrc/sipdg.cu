@@ -121,6 +121,8 @@ int setup_grad(dgop_operator* op, KronDiffCfg<double>& K) {
   return DGOP_OK;
 }
 
+constexpr int64_t kDiffSmall = 2048;  // elements; setup_diff3d
+
 // The 3D register kernel's launch (kron3d_diff_kernel.cuh), where it covers the order; leaves entry3d
 // null otherwise.
 template <typename Real>
@@ -182,6 +184,10 @@ int setup_diff3d(dgop_operator* op, KronDiffCfg<Real>& K, const std::vector<doub
     K.grid3d[mode] = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((groups + warps - 1) / warps, sms * per_sm)));
   }
   K.entry3d = entry;
+  // Small meshes at p = 5 in FP64: a warp's group of five elements is one long chain at 255 registers, and
+  // below three waves of groups the shared-memory kernel, with 256 threads, is the faster (us, register /
+  // shared memory: 15.5 / 15.0 at 12^3 elements, 14.9 / 12.1 at 8^3, 15.9 / 18.8 at 13^3).
+  K.apply3d = !(N == 6 && sizeof(Real) == 8 && s.nelem < kDiffSmall);
   return DGOP_OK;
 }
 
