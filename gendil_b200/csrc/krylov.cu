@@ -303,6 +303,7 @@ __global__ void k_gm_backsub(const GMState* st, const double* H, const double* e
 // ---------------------------------------------- GMRES with iterative refinement (inner basis)
 
 constexpr int kGsChunk = 16;    // basis vectors per block row of the projection pass
+constexpr int kGsSmallChunk = 8;  // the same on small systems (k_gs_dots_small)
 constexpr int kGsMaxRestart = 1000;
 
 template <typename T>
@@ -400,6 +401,42 @@ __global__ void __launch_bounds__(kRT, 2) k_gs_dots(const GMState* st, const T* 
     DGOP_GS_CASE(13) DGOP_GS_CASE(14) DGOP_GS_CASE(15) DGOP_GS_CASE(16)
 #undef DGOP_GS_CASE
   }
+}
+
+// The same for systems that leave a thread at most one access per vector: one code for every number of
+// vectors.  There the compiled widths above cost more than their loads gain, since a restart cycle runs
+// another one, fetched anew, in every step (us per step of a restart of 60 in FP64, 1728 / 110,592 / 2.3 M
+// dofs: this one 41.6 / 45.9 / 259.8, the other 46.5 / 48.8 / 252.0).
+template <typename T>
+__global__ void __launch_bounds__(kRT) k_gs_dots_small(const GMState* st, const T* __restrict__ V, int64_t ld, int j,
+                                                       const T* __restrict__ w, double* wide) {
+  if (st->inactive) return;
+  using V16 = typename Vec16<T>::type;
+  constexpr int L = Vec16<T>::L, C = kGsSmallChunk;
+  const int i0 = blockIdx.y * C;
+  const int cnt = min(C, j + 1 - i0);
+  double acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) acc[c] = 0.0;
+  const int64_t nv = ld / L;
+  const V16* w16 = reinterpret_cast<const V16*>(w);
+  const V16* v16 = reinterpret_cast<const V16*>(V + (int64_t)i0 * ld);
+  DGOP_GRID_LOOP(u, nv) {
+    T wv[L];
+    *reinterpret_cast<V16*>(wv) = w16[u];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      if (c < cnt) {
+        T vv[L];
+        *reinterpret_cast<V16*>(vv) = v16[c * nv + u];
+#pragma unroll
+        for (int k = 0; k < L; ++k) acc[c] += (double)vv[k] * (double)wv[k];
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (c < cnt) write_partial(wide + (int64_t)(i0 + c) * kRB, acc[c]);
 }
 
 // H(i, j) <- (V_i, w), one block per i, partials summed in the fixed order
@@ -923,8 +960,10 @@ int gmres_ir_solve(SolverImpl& s, const double* b, double* x, int max_iters, dou
       } else {
         DGOP_TRY(apply_op(vj, w, q));
       }
-      const dim3 dgrid(kRB, (j + 1 + kGsChunk - 1) / kGsChunk);
-      k_gs_dots<T><<<dgrid, kRT, 0, q>>>(gs, V, ld, j, w, s.wide);
+      if (ld / Vec16<T>::L <= (int64_t)kRB * kRT)
+        k_gs_dots_small<T><<<dim3(kRB, j / kGsSmallChunk + 1), kRT, 0, q>>>(gs, V, ld, j, w, s.wide);
+      else
+        k_gs_dots<T><<<dim3(kRB, j / kGsChunk + 1), kRT, 0, q>>>(gs, V, ld, j, w, s.wide);
       k_gs_h<<<j + 1, kRT, 0, q>>>(gs, j, m, H, s.wide);
       k_gs_update<T><<<kRB, kRT, 0, q>>>(gs, V, ld, j, m, H, w, vn, pa);
       k_gm_column<<<1, kRT, 0, q>>>(gs, j, m, H, csv, snv, e1, pa);
