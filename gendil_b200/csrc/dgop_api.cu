@@ -612,31 +612,25 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
                                                            : K.factors && kron_early_factors(N) ? kv.warp_smem_fact
                                                                                                 : kv.warp_smem);
     if ((int)L.smem > max_smem - 1024) continue;  // 1 KB covers every variant's static shared memory
-    int arc = allow_dynamic_smem(kv.func, max_smem);
-    if (arc == DGOP_OK) arc = allow_dynamic_smem(kv.func_sep, max_smem);
-    for (const void* f : kv.func_dot)
-      if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
-    for (const auto& by_sep : kv.func_general)
-      for (const void* f : by_sep)
-        if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
-    for (const auto& by_dot : kv.func_masked)
-      for (const auto& by_sep : by_dot)
-        for (const void* f : by_sep)
-          if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
-    for (const auto& by_dot : kv.func_fact)
-      for (const auto& by_sep : by_dot)
-        for (const void* f : by_sep)
-          if (arc == DGOP_OK && f) arc = allow_dynamic_smem(f, max_smem);
-    if (arc != DGOP_OK) return arc;
-    // resident CTAs per SM of the kernels this operator launches (the slot-mask form when its
-    // mask has one), plain and with the inner-product epilogue: each gets a grid of that many
-    const int mi = kron_mask_index(p);
-    const void* kern[2] = {sep ? kv.func_sep : kv.func, kv.func_dot[sep ? 1 : 0]};
-    for (int dot = 0; dot < 2; ++dot)
-      if (p.general) kern[dot] = kv.func_general[dot][sep ? 1 : 0];
-      else if (K.factors && kv.func_fact[dot][sep ? 1 : 0][mi + 1]) kern[dot] = kv.func_fact[dot][sep ? 1 : 0][mi + 1];
-      else if (K.factors && kv.func_fact[dot][sep ? 1 : 0][0]) kern[dot] = kv.func_fact[dot][sep ? 1 : 0][0];
-      else if (mi >= 0 && kv.func_masked[mi][dot][sep ? 1 : 0]) kern[dot] = kv.func_masked[mi][dot][sep ? 1 : 0];
+    // the kernels this operator launches, plain and with the inner-product epilogue: the general form,
+    // or the slot-mask form where the mask (of the transposed operator its own) has one
+    auto kernel_of = [&](const KronParams<Real>& q, int dot) -> const void* {
+      if (p.general) return kv.func_general[dot][sep ? 1 : 0];
+      const int mi = kron_mask_index(q);
+      if (K.factors)
+        for (int i : {mi + 1, 0})
+          if (kv.func_fact[dot][sep ? 1 : 0][i]) return kv.func_fact[dot][sep ? 1 : 0][i];
+      if (mi >= 0 && kv.func_masked[mi][dot][sep ? 1 : 0]) return kv.func_masked[mi][dot][sep ? 1 : 0];
+      return dot ? kv.func_dot[sep ? 1 : 0] : sep ? kv.func_sep : kv.func;
+    };
+    const void* kern[2] = {kernel_of(p, 0), kernel_of(p, 1)};
+    for (int dot = 0; dot < 2; ++dot) {
+      const void* other = kernel_of(K.params_t, dot);
+      int arc = kern[dot] ? allow_dynamic_smem(kern[dot], max_smem) : DGOP_OK;
+      if (arc == DGOP_OK && other && other != kern[dot]) arc = allow_dynamic_smem(other, max_smem);
+      if (arc != DGOP_OK) return arc;
+    }
+    // resident CTAs per SM of each: grids of that many
     int per_sm = 0, per_sm_dot = 0;
     DGOP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern[0], threads, L.smem));
     if (per_sm < 1) continue;
