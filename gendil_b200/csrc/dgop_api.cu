@@ -428,13 +428,35 @@ int allow_dynamic_smem(const void* f, int max_smem) {
   return DGOP_OK;
 }
 
+// Device tables of an operator in one allocation and one copy: sections of Reals and of signs, each at a
+// multiple of 128 bytes (a cache line).
 template <typename Real>
-int upload(Real** dst, const double* src, size_t n) {
-  std::vector<Real> tmp(src, src + n);
-  DGOP_CUDA(cudaMalloc(dst, sizeof(Real) * (n ? n : 1)));
-  if (n) DGOP_CUDA(cudaMemcpy(*dst, tmp.data(), sizeof(Real) * n, cudaMemcpyHostToDevice));
-  return DGOP_OK;
-}
+struct TableUpload {
+  std::vector<unsigned char> bytes;
+  size_t reals(const double* src, size_t n) {
+    const size_t at = section(sizeof(Real) * n);
+    Real* d = reinterpret_cast<Real*>(bytes.data() + at);
+    for (size_t i = 0; i < n; ++i) d[i] = (Real)src[i];
+    return at;
+  }
+  size_t signs(const signed char* src, size_t n) {
+    const size_t at = section(n);
+    if (n) std::memcpy(bytes.data() + at, src, n);
+    return at;
+  }
+  int send(unsigned char** dst) const {
+    DGOP_CUDA(cudaMalloc(dst, bytes.size() ? bytes.size() : 16));
+    if (!bytes.empty()) DGOP_CUDA(cudaMemcpy(*dst, bytes.data(), bytes.size(), cudaMemcpyHostToDevice));
+    return DGOP_OK;
+  }
+
+ private:
+  size_t section(size_t n) {
+    const size_t at = bytes.size();
+    bytes.resize(at + (n + 127) / 128 * 128);
+    return at;
+  }
+};
 
 template <typename Real>
 int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, const double* elem_sigma,
@@ -469,9 +491,27 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
     for (int i = 0; i < s.n; ++i) p.lf[f][i] = (Real)face_values[f][i];
   for (int t = 0; t < plan.nextra; ++t)
     for (int k = 0; k < 3; ++k) p.extra[t][k] = plan.extra[t][k];
-  int rc = upload<Real>(&K.d_mats, plan.mats.data(), plan.mats.size());
+  TableUpload<Real> tables;
+  const size_t mats_at = tables.reals(plan.mats.data(), plan.mats.size());
+  size_t phi_at = 0, sgn_at = 0;
+  size_t phi_off[3] = {}, sg_off[3][3] = {};
+  if (plan.has_adv) {
+    std::vector<double> phi;
+    std::vector<signed char> sg;
+    for (int a = 0; a < 3; ++a) {
+      phi_off[a] = phi.size();
+      phi.insert(phi.end(), plan.phi[a].begin(), plan.phi[a].end());
+      for (int k = 0; k < 3; ++k) {
+        sg_off[a][k] = sg.size();
+        sg.insert(sg.end(), plan.sgn[a][k].begin(), plan.sgn[a][k].end());
+      }
+    }
+    phi_at = tables.reals(phi.data(), phi.size());
+    sgn_at = tables.signs(sg.data(), sg.size());
+  }
+  int rc = tables.send(&K.d_tables);
   if (rc) return rc;
-  p.mats = K.d_mats;
+  p.mats = reinterpret_cast<const Real*>(K.d_tables + mats_at);
   // slot -> matrix table; constant tables go to kernel-parameter space
   const int N = s.n;
   // the kernel reads element-dependent matrices with vector loads when N allows them
@@ -503,24 +543,10 @@ int setup_kron(dgop_operator* op, KronCfg<Real>& K, const KronPlanHost& plan, co
       put(p, kSlotMX, plan.MT[0]);
       put(p, kSlotMY, plan.MT[1]);
     }
-    std::vector<double> phi;
-    std::vector<signed char> sg;
-    size_t phi_off[3], sg_off[3][3];
     for (int a = 0; a < 3; ++a) {
-      phi_off[a] = phi.size();
-      phi.insert(phi.end(), plan.phi[a].begin(), plan.phi[a].end());
-      for (int k = 0; k < 3; ++k) {
-        sg_off[a][k] = sg.size();
-        sg.insert(sg.end(), plan.sgn[a][k].begin(), plan.sgn[a][k].end());
-      }
-    }
-    rc = upload<Real>(&K.d_phi, phi.data(), phi.size());
-    if (rc) return rc;
-    DGOP_CUDA(cudaMalloc(&K.d_sgn, sg.size() ? sg.size() : 1));
-    if (!sg.empty()) DGOP_CUDA(cudaMemcpy(K.d_sgn, sg.data(), sg.size(), cudaMemcpyHostToDevice));
-    for (int a = 0; a < 3; ++a) {
-      p.phi[a] = K.d_phi + phi_off[a];
-      for (int k = 0; k < 3; ++k) p.sgn[a][k] = (k == a) ? nullptr : K.d_sgn + sg_off[a][k];
+      p.phi[a] = reinterpret_cast<const Real*>(K.d_tables + phi_at) + phi_off[a];
+      for (int k = 0; k < 3; ++k)
+        p.sgn[a][k] = k == a ? nullptr : reinterpret_cast<const signed char*>(K.d_tables + sgn_at) + sg_off[a][k];
     }
   } else if (!plan.nextra) {
     put(p, kSlotDZ, plan.MD);
@@ -911,19 +937,14 @@ int setup_kronnd(dgop_operator* op, KronNDCfg<Real>& K, const KronPlanHost& plan
   p.has_mass = plan.has_mass;
   p.mass_merged = plan.mass_merged;
   p.g = (Real)op->g;
-  int rc = upload<Real>(&K.d_mats, plan.mats.data(), plan.mats.size());
-  if (rc) return rc;
-  p.mats = K.d_mats;
-  for (int a = 0; a < kMaxDim; ++a) {
-    for (int k = 0; k < kMaxDim; ++k) p.slot[a][k] = KronMat{};
-    p.mslot[a] = KronMat{};
-  }
+  TableUpload<Real> tables;
+  const size_t mats_at = tables.reals(plan.mats.data(), plan.mats.size());
+  size_t phi_at = 0, sgn_at = 0, pmats_at = 0;
+  size_t phi_off[kMaxDim] = {}, sg_off[kMaxDim][kMaxDim] = {};
+  const bool split = entry->func_s && plan.has_adv;  // the split variant (5): operators with advection terms
   if (plan.has_adv) {
-    for (int a = 0; a < D; ++a)
-      for (int k = 0; k < D; ++k) p.slot[a][k] = (k == a) ? plan.D[a] : plan.T[a][k];
     std::vector<double> phi;
     std::vector<signed char> sg;
-    size_t phi_off[kMaxDim], sg_off[kMaxDim][kMaxDim];
     for (int a = 0; a < D; ++a) {
       phi_off[a] = phi.size();
       phi.insert(phi.end(), plan.phi[a].begin(), plan.phi[a].end());
@@ -932,13 +953,30 @@ int setup_kronnd(dgop_operator* op, KronNDCfg<Real>& K, const KronPlanHost& plan
         sg.insert(sg.end(), plan.sgn[a][k].begin(), plan.sgn[a][k].end());
       }
     }
-    rc = upload<Real>(&K.d_phi, phi.data(), phi.size());
-    if (rc) return rc;
-    DGOP_CUDA(cudaMalloc(&K.d_sgn, sg.size() ? sg.size() : 1));
-    if (!sg.empty()) DGOP_CUDA(cudaMemcpy(K.d_sgn, sg.data(), sg.size(), cudaMemcpyHostToDevice));
+    phi_at = tables.reals(phi.data(), phi.size());
+    sgn_at = tables.signs(sg.data(), sg.size());
+  }
+  if (split) {
+    const int matp = entry->split_matp, mat = N * N;
+    std::vector<double> padded(plan.mats.size() / mat * matp, 0.0);
+    for (size_t m = 0; m < plan.mats.size() / mat; ++m)
+      std::copy_n(plan.mats.begin() + m * mat, mat, padded.begin() + m * matp);
+    pmats_at = tables.reals(padded.data(), padded.size());
+  }
+  int rc = tables.send(&K.d_tables);
+  if (rc) return rc;
+  p.mats = reinterpret_cast<const Real*>(K.d_tables + mats_at);
+  for (int a = 0; a < kMaxDim; ++a) {
+    for (int k = 0; k < kMaxDim; ++k) p.slot[a][k] = KronMat{};
+    p.mslot[a] = KronMat{};
+  }
+  if (plan.has_adv) {
+    for (int a = 0; a < D; ++a)
+      for (int k = 0; k < D; ++k) p.slot[a][k] = (k == a) ? plan.D[a] : plan.T[a][k];
     for (int a = 0; a < D; ++a) {
-      p.phi[a] = K.d_phi + phi_off[a];
-      for (int k = 0; k < D; ++k) p.sgn[a][k] = (k == a) ? nullptr : K.d_sgn + sg_off[a][k];
+      p.phi[a] = reinterpret_cast<const Real*>(K.d_tables + phi_at) + phi_off[a];
+      for (int k = 0; k < D; ++k)
+        p.sgn[a][k] = k == a ? nullptr : reinterpret_cast<const signed char*>(K.d_tables + sgn_at) + sg_off[a][k];
     }
   }
   if (plan.has_mass && !(plan.has_adv && plan.mass_merged)) {
@@ -1032,16 +1070,10 @@ int setup_kronnd(dgop_operator* op, KronNDCfg<Real>& K, const KronPlanHost& plan
     const int64_t cv = std::min<int64_t>((s.nelem + ebv - 1) / ebv, (int64_t)device_sm_count(op->device) * per_sm_v);
     K.var[v] = {true, ebv, dim3((unsigned)std::max<int64_t>(cv, 1)), pv * ebv + extra, 0.0f, threads};
   }
-  // the split variant (5): operators with advection terms
-  if (entry->func_s && plan.has_adv) {
-    const int matp = entry->split_matp, mat = N * N;
-    std::vector<double> padded(plan.mats.size() / mat * matp, 0.0);
-    for (size_t m = 0; m < plan.mats.size() / mat; ++m)
-      std::copy_n(plan.mats.begin() + m * mat, mat, padded.begin() + m * matp);
-    rc = upload<Real>(&K.d_pmats, padded.data(), padded.size());
-    if (rc) return rc;
+  if (split) {
+    const int mat = N * N;
     for (KronNDParams<Real>* q : {&p, &K.params_t}) {
-      q->pmats = K.d_pmats;
+      q->pmats = reinterpret_cast<const Real*>(K.d_tables + pmats_at);
       for (int a = 0; a <= D; ++a)
         for (int k = 0; k < D; ++k) {
           const KronMat m = a < D ? q->slot[a][k] : q->mslot[k];
@@ -1181,10 +1213,7 @@ template <typename Real>
 void free_kronnd(KronNDCfg<Real>& K) {
   if (K.d_tc_tiles) cudaFree(K.d_tc_tiles);
   if (K.d_tc_scale) cudaFree(K.d_tc_scale);
-  if (K.d_pmats) cudaFree(K.d_pmats);
-  if (K.d_mats) cudaFree(K.d_mats);
-  if (K.d_phi) cudaFree(K.d_phi);
-  if (K.d_sgn) cudaFree(K.d_sgn);
+  if (K.d_tables) cudaFree(K.d_tables);
   for (auto* p : K.d_elem)
     if (p) cudaFree(p);
   K = KronNDCfg<Real>{};
@@ -1193,9 +1222,7 @@ void free_kronnd(KronNDCfg<Real>& K) {
 template <typename Real>
 void free_kron(KronCfg<Real>& K) {
   if (K.d_tma) cudaFree(K.d_tma);
-  if (K.d_mats) cudaFree(K.d_mats);
-  if (K.d_phi) cudaFree(K.d_phi);
-  if (K.d_sgn) cudaFree(K.d_sgn);
+  if (K.d_tables) cudaFree(K.d_tables);
   for (auto* p : K.d_elem)
     if (p) cudaFree(p);
   K = KronCfg<Real>{};

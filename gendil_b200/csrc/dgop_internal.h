@@ -50,9 +50,7 @@ struct KronCfg {
   } launch[kKronVariants];
   int variant = 0;  // the kernel variant in use
   int fallback = 1;  // fastest variant without bulk-tensor staging (element ranges not in whole groups)
-  Real* d_mats = nullptr;
-  Real* d_phi = nullptr;
-  signed char* d_sgn = nullptr;
+  unsigned char* d_tables = nullptr;  // matrices, face coefficients and their signs
   Real* d_elem[4] = {};  // converted per-element factors (FP32 only)
   bool factors = false;  // per-element velocity factors
   // bulk-tensor variants: face words per element and slot words per group of 8 elements, for the
@@ -81,9 +79,7 @@ struct KronNDCfg {
   KronNDParams<Real> params_t{};  // transposed operator
   dim3 grid, block;
   size_t smem = 0;
-  Real* d_mats = nullptr;
-  Real* d_phi = nullptr;
-  signed char* d_sgn = nullptr;
+  unsigned char* d_tables = nullptr;  // matrices, face coefficients and their signs
   Real* d_elem[kMaxDim + 1] = {};  // converted per-element factors (FP32 only)
   // launch shapes of the variants (kKronNDVariants; 0 = grid / smem / params.eb above)
   struct Variant {
@@ -96,7 +92,6 @@ struct KronNDCfg {
   } var[kKronNDVariants];
   int variant = 0;
   bool preferred = false;   // a 3D register-kernel operator's applies run here
-  Real* d_pmats = nullptr;  // the split variant's padded matrix table
   // BF16 tensor-core launch (FP32 configuration only) and its Kronecker tile tables
   bool tc_ok = false;
   dim3 tc_grid;
