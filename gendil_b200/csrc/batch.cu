@@ -76,12 +76,28 @@ void release(dgop_batch* b) {
   if (b->applied) cudaEventDestroy(b->applied);
 }
 
+// The split variant's own launch prefetches its elements and reads its parameters from constant memory, the
+// batch kernel does neither, so a group pays where the launches it saves (5 to 7 us of the host each) outweigh
+// that: members up to about 3 us of kernel, four of them at least, in a batch that keeps the host busier
+// than the GPU (below about 300,000 dofs per launch, 5 us at 60 GDoF/s; 24 systems of 671,000 dofs on
+// average 218 one launch each, 228 with its two small groups).  Us per batched apply, one launch
+// each / grouped: 32 systems of 2D p = 3, 128,000 dofs 158 / 99, 320,000 dofs 171 / 208; of 2D p = 5,
+// 144,000 dofs 167 / 158, 288,000 dofs 194 / 287; 4D p = 2, 81,000 dofs (64 systems) 326 / 205, 324,000
+// dofs 268 / 289; 512 of 2D p = 2, 9,000 dofs 2514 / 1119.  (2D p = 1: grouped from two members on, up to the
+// limit of the other variants.)
+constexpr int64_t kSplitGroupDofs = 200000;
+constexpr size_t kSplitGroupMembers = 4;
+constexpr int64_t kSplitMeanDofs = 300000;
+
 int setup(dgop_batch* b) {
   int sms = 0, dev = 0;
   DGOP_CUDA_B(cudaGetDevice(&dev));
   DGOP_CUDA_B(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   int max_smem = 0;
   DGOP_CUDA_B(cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  int64_t mean = 0;  // dofs per operator
+  for (const dgop_operator* op : b->ops) mean += op->sp.ndofs;
+  mean /= (int64_t)b->ops.size();
   std::map<const void*, int> per_sm_of;  // resident CTAs per SM of each batch kernel used
   std::map<std::tuple<int, int, int>, int> index;
   for (int i = 0; i < (int)b->ops.size(); ++i) {
@@ -107,7 +123,8 @@ int setup(dgop_batch* b) {
     // parameters in constant memory, no per-batch instance lookup): the persistent kernel gains
     // nothing there and measured a few per cent slower
     const int64_t eb = op->n64.var[v].eb;
-    if ((op->sp.nelem + eb - 1) / eb >= 2 * (int64_t)sms * pit->second) {
+    const bool split = v == 5 && !(op->sp.D == 2 && op->sp.n == 2);
+    if ((op->sp.nelem + eb - 1) / eb >= 2 * (int64_t)sms * pit->second || (split && (op->sp.ndofs > kSplitGroupDofs || mean > kSplitMeanDofs))) {
       b->singles.push_back(i);
       continue;
     }
@@ -125,10 +142,12 @@ int setup(dgop_batch* b) {
     BatchGroup& group = b->groups[it->second];
     group.members.push_back(i);
   }
-  // a lone operator of the split variant keeps its own launch, which prefetches its elements
+  // few operators of the split variant keep their own launches
   for (size_t k = 0; k < b->groups.size();) {
-    if (b->groups[k].variant == 5 && b->groups[k].members.size() == 1) {
-      b->singles.push_back(b->groups[k].members[0]);
+    const auto& m = b->groups[k].members;
+    const dgop_space& sp = b->ops[m[0]]->sp;
+    if (b->groups[k].variant == 5 && m.size() < (sp.D == 2 && sp.n == 2 ? 2 : kSplitGroupMembers)) {
+      b->singles.insert(b->singles.end(), m.begin(), m.end());
       b->groups.erase(b->groups.begin() + (long)k);
     } else {
       ++k;

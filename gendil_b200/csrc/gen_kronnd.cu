@@ -120,7 +120,7 @@ void fill(KronNDEntry<Real>& d) {
       d.split_warp_bytes = SplitShape<D, N>::template warp_bytes<Real>();
       d.split_epw = SplitShape<D, N>::EPW;
       d.split_matp = split_matp<N, Real>();
-      if constexpr (D == 2 && N == 2 && sizeof(Real) == 8) {
+      if constexpr (sizeof(Real) == 8) {
         d.launch_batch[5] = &launch_kronnd_split_batch<D, N, Real>;
         d.func_batch[5] = reinterpret_cast<const void*>(&kronnd_split_batch_kernel<D, N, Real>);
       }

@@ -261,3 +261,28 @@ def test_batch_with_a_repeated_operator_that_owns_a_workspace():
         torch.cuda.synchronize()
         assert all(torch.equal(a, b) for a, b in zip(want, ys))
     batch.close()
+
+
+@pytest.mark.parametrize("D,p,count,n", [(2, 1, 60, 60), (2, 2, 12, 60), (2, 5, 6, 40), (2, 7, 4, 20), (4, 1, 6, 6),
+                                         (4, 3, 4, 4), (6, 1, 4, 3), (6, 2, 4, 2)])
+def test_split_variant_groups(D, p, count, n):
+    """Groups of the split variant, with more element batches than the batch kernel has CTAs for the small
+    orders (a CTA moves from one instance to the next and takes its matrices), extents that differ
+    from instance to instance, and velocities that vary along an axis in every other one."""
+    rng = np.random.default_rng(D * 10 + p)
+    ops = []
+    for i in range(count):
+        sp = _space(D, [n + i % 3] + [n] * (D - 1), p)
+        beta = C.velocity_sincos(D) if i % 2 else C.velocity_constant(list(rng.uniform(-1, 1, D)))
+        o = g.SystemOperator(sp, min(8, p + 2), beta, sigma=1e3)
+        o.set_variant("nd-split")
+        ops.append(o)
+    xs = [torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops]
+    want = [o(x, torch.empty_like(x)) for o, x in zip(ops, xs)]
+    batch = g.Batch(ops)
+    assert batch.groups == 1
+    ys = [torch.full_like(x, float("nan")) for x in xs]
+    batch.apply(xs, ys)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(want, ys))
+    batch.close()
