@@ -327,19 +327,24 @@ __device__ __forceinline__ void memory_pass(const Real* p, Real (&X)[N][N]) {
     lines_inplace_rows<N, FIRST>(p, X);
   }
 }
-// Y <- A X along the second plane index, or Y += with ACC, A in memory at p.
+// Y <- A X along the second plane index, or Y += with ACC, A in memory at p.  In FP64 the products accumulate
+// onto Y in one multiply-add chain per value.  In FP32 a term is summed on its own and then added: the
+// chain rounds every product at the size of the whole sum, which made the applies' error up to a
+// quarter larger (advection against 64 bits, p = 3 / p = 5: chained 1.03e-7 / 1.19e-7, own sums 0.90e-7 /
+// 0.97e-7; 48^3 p = 3 takes 26.6 us instead of 26.2).  In FP64 the two differ by less than 0.2 %.
 template <int N, bool ACC, typename Real>
 __device__ __forceinline__ void memory_pass_z(const Real* p, const Real (&X)[N][N], Real (&Y)[N][N]) {
+  constexpr bool chain = ACC && sizeof(Real) == 8;
 #pragma unroll
   for (int k = 0; k < N; ++k) {
     Real row[N];
     matrix_row<N>(p, k, row);
 #pragma unroll
     for (int i = 0; i < N; ++i) {
-      Real s = ACC ? Y[i][k] : Real(0);
+      Real s = chain ? Y[i][k] : row[0] * X[i][0];
 #pragma unroll
-      for (int r = 0; r < N; ++r) s = (!ACC && r == 0) ? row[0] * X[i][0] : s + row[r] * X[i][r];
-      Y[i][k] = s;
+      for (int r = chain ? 0 : 1; r < N; ++r) s += row[r] * X[i][r];
+      Y[i][k] = ACC && !chain ? Y[i][k] + s : s;
     }
   }
 }
@@ -354,11 +359,11 @@ __device__ __forceinline__ void kron_pass(const Block& P, uint32_t coord, Real (
   }
 }
 
-// Y <- (slot SLOT's matrix) X along the second plane index, or Y += with ACC (the products
-// accumulate onto Y in one multiply-add chain per value).
+// Y <- (slot SLOT's matrix) X along the second plane index, or Y += with ACC (summed as in memory_pass_z).
 template <int N, typename Real, int SLOT, bool ACC, uint32_t VM, typename Block>
 __device__ __forceinline__ void kron_pass_z(const Block& P, uint32_t coord, const Real (&X)[N][N],
                                             Real (&Y)[N][N]) {
+  [[maybe_unused]] constexpr bool chain = ACC && sizeof(Real) == 8;
   if (slot_varies<SLOT, VM>(P)) {
     memory_pass_z<N, ACC>(slot_matrix<SLOT>(P, coord), X, Y);
   } else {
@@ -367,10 +372,10 @@ __device__ __forceinline__ void kron_pass_z(const Block& P, uint32_t coord, cons
     for (int k = 0; k < N; ++k)
 #pragma unroll
       for (int i = 0; i < N; ++i) {
-        Real s = ACC ? Y[i][k] : Real(0);
+        Real s = chain ? Y[i][k] : A(k, 0) * X[i][0];
 #pragma unroll
-        for (int r = 0; r < N; ++r) s = (!ACC && r == 0) ? A(k, 0) * X[i][0] : s + A(k, r) * X[i][r];
-        Y[i][k] = s;
+        for (int r = chain ? 0 : 1; r < N; ++r) s += A(k, r) * X[i][r];
+        Y[i][k] = ACC && !chain ? Y[i][k] + s : s;
       }
   }
 }

@@ -160,3 +160,21 @@ def test_gauss_legendre_mass_takes_the_faster_kernel(D, p, kernel):
     y, y32 = cuda_apply(op, x), cuda_apply(op, x, f32=True)
     op.select_kernel("generic")
     assert rel_max(y, cuda_apply(op, x)) <= APPLY_TOL and rel_max(y32, y) <= 1e-5
+
+
+@pytest.mark.parametrize("p", range(1, 6))
+def test_fp32_rounding_of_the_register_kernel(p):
+    """The FP32 apply's error (2-norm, against the FP64 apply) is that of the any-dimension kernel, which
+    contracts axis by axis and adds whole terms: the same roundings in another order, which move a norm
+    over 10^4 values and more by a few per cent.  (Terms summed onto one another's partial sums, at
+    the size of all of them, take 6 to 21 % more.)"""
+    sp = g.Space(3, [11, 10, 9], order=p)
+    op = g.AdvectionOperator(sp, p + 1, C.velocity_sincos(3))
+    assert op.kernel == "kron", op.kernel_note
+    x = np.random.default_rng(p).uniform(-1, 1, sp.num_dofs).astype(np.float32).astype(np.float64)
+    y = cuda_apply(op, x)
+    err = []
+    for kernel in ("kron", "kronnd"):
+        op.select_kernel(kernel)
+        err.append(np.linalg.norm(cuda_apply(op, x, f32=True) - y))
+    assert err[0] <= 1.05 * err[1], err
