@@ -69,3 +69,45 @@ def test_cg_with_fused_product_matches_separate_pass():
     assert torch.equal(got[0][0], got[1][0]) and got[0][1] == got[1][1]
     # the same products in another fixed order: iterates agree to the stopping tolerance
     assert rel_max(got[0][0].cpu().numpy(), got[2][0].cpu().numpy()) <= 1e-8
+
+
+@pytest.mark.parametrize("p", range(1, 6))
+def test_gauss_legendre_with_a_wrapped_x_axis(p):
+    """Wrapped x neighbours, which are not in the staged group, on a basis whose traces are whole lines: the
+    apply and the coefficient gradient, FP32, and CG with the fused inner product (p = 5 has none on a mesh
+    this small: its apply is the shared-memory kernel's)."""
+    sp = g.Space(3, [32 // (p + 1) + 2, 2, 3], [0.3, 0.2, 0.5], None, [1, 0, 0], p, g.GL)
+    gen = torch.Generator(device="cuda").manual_seed(p)
+    rand = lambda n: torch.rand(n, dtype=torch.float64, device="cuda", generator=gen) - 0.5  # noqa: E731
+    mu = torch.exp(rand(sp.num_elements))
+    op = g.SIPDGOperator(sp, p + 1, mu)
+    x, lam = rand(sp.num_dofs), rand(sp.num_dofs)
+    y, want = op(x, torch.empty_like(x)), op(_offset(x), _offset(x))
+    scale = float(want.abs().max())
+    assert float((y - want).abs().max()) <= 1e-13 * scale
+    z = op.apply_f32(x.float(), torch.empty(sp.num_dofs, dtype=torch.float32, device="cuda"))
+    assert float((z.double() - want).abs().max()) <= 1e-5 * scale
+    grad, gwant = op.coefficient_gradient(x, lam), op.coefficient_gradient(_offset(x), lam)
+    assert float((grad - gwant).abs().max()) <= 1e-13 * max(float(gwant.abs().max()), scale)
+    got = []
+    for fused in (True, False):
+        u = torch.zeros_like(x)
+        assert g.CGSolver(op).fused_dot(fused).solve(x, u, 5000, 1e-10)["success"]
+        got.append(u)
+    # the same products in another fixed order: iterates agree to the stopping tolerance
+    assert rel_max(got[0].cpu().numpy(), got[1].cpu().numpy()) <= 1e-8
+
+
+@pytest.mark.parametrize("elements", [12 * 13 * 13, 13 * 13 * 13])
+def test_order_5_apply_on_either_side_of_the_small_mesh_limit(elements):
+    """Below 2048 elements the FP64 apply at p = 5 is the shared-memory kernel's, bit for bit that of vectors off
+    16 bytes; above, the register kernel's, which sums in another order."""
+    sizes = [elements // 169, 13, 13]
+    sp = g.Space(3, sizes, order=5)
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda n: torch.rand(n, dtype=torch.float64, device="cuda", generator=gen) - 0.5  # noqa: E731
+    op = g.SIPDGOperator(sp, 6, torch.exp(rand(sp.num_elements)))
+    x = rand(sp.num_dofs)
+    y, off = op(x, torch.empty_like(x)), op(_offset(x), _offset(x))
+    assert torch.equal(y, off) == (elements < 2048)
+    assert float((y - off).abs().max()) <= 1e-13 * float(off.abs().max())

@@ -178,3 +178,21 @@ def test_fp32_rounding_of_the_register_kernel(p):
         op.select_kernel(kernel)
         err.append(np.linalg.norm(cuda_apply(op, x, f32=True) - y))
     assert err[0] <= 1.05 * err[1], err
+
+
+@pytest.mark.parametrize("basis", [g.GLL, g.GL])
+@pytest.mark.parametrize("p", [1, 2, 3, 4, 5])
+def test_system_with_a_density_that_is_a_sum(p, basis):
+    """Advection terms and the mass terms of a sum of products in one launch, with a per-element density
+    factor: forward, transposed and FP32, against the generic kernel."""
+    sp = g.Space(3, [32 // (p + 1) + 1, 2, 3], order=p, basis=basis)
+    factor = torch.from_numpy(np.random.default_rng(p).uniform(0.5, 1.5, sp.num_elements)).cuda()
+    density = C.density_poly(3)
+    sigma = C.Coefficient(constant=density.constant, terms=density.terms, element_factor=factor)
+    op = g.SystemOperator(sp, p + 2, C.velocity_sincos(3), sigma=sigma, bc=g.BC_INFLOW, g=0.3)
+    assert op.kernel == "kron", op.kernel_note
+    x = np.random.default_rng(p + 1).uniform(-1, 1, sp.num_dofs)
+    y, yt, y32 = cuda_apply(op, x), cuda_apply(op, x, transpose=True), cuda_apply(op, x, f32=True)
+    op.select_kernel("generic")
+    assert rel_max(y, cuda_apply(op, x)) <= APPLY_TOL and rel_max(yt, cuda_apply(op, x, transpose=True)) <= APPLY_TOL
+    assert rel_max(y32, y) <= 1e-5
