@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <map>
 #include <new>
 #include <numeric>
 #include <vector>
@@ -368,13 +369,16 @@ int setup(dgop_batch_solver* s, double budget_bytes) {
 }
 
 // Run body(k, stream) for every system k of a wave, spread over the branch streams after a fork
-// from q and joined back into q (inside a capture these become parallel graph branches).
+// from q and joined back into q (inside a capture these become parallel graph branches).  alone[k]: the
+// system applies an operator that others of the wave apply too and whose applies share memory; these
+// systems take one branch, in turn.
 template <typename F>
-int per_system(dgop_batch_solver* s, int count, cudaStream_t q, F&& body) {
+int per_system(dgop_batch_solver* s, const std::vector<char>& alone, cudaStream_t q, F&& body) {
+  const int count = (int)alone.size();
   const int nb = std::min(count, 16);
   DGOP_CUDA_BS(cudaEventRecord(s->fork, q));
   for (int k = 0; k < nb; ++k) DGOP_CUDA_BS(cudaStreamWaitEvent(s->branch[k], s->fork, 0));
-  for (int k = 0; k < count; ++k) DGOP_TRY_BS(body(k, s->branch[k % nb]));
+  for (int k = 0; k < count; ++k) DGOP_TRY_BS(body(k, s->branch[alone[k] ? 0 : k % nb]));
   for (int k = 0; k < nb; ++k) {
     DGOP_CUDA_BS(cudaEventRecord(s->join[k], s->branch[k]));
     DGOP_CUDA_BS(cudaStreamWaitEvent(q, s->join[k], 0));
@@ -397,6 +401,15 @@ int solve_wave(dgop_batch_solver* s, const std::vector<int>& wave, const double*
   const int m = s->restart;
   const int count = (int)wave.size();
   const int pw = m + 1;
+  std::map<const dgop_operator*, int> uses;
+  for (int i : wave) {
+    ++uses[s->ops[i]];
+    if (s->precs[i]) ++uses[s->precs[i]];
+  }
+  std::vector<char> alone(count, 0);
+  for (int k = 0; k < count; ++k)
+    for (const dgop_operator* op : {s->ops[wave[k]], s->precs[wave[k]]})
+      if (op && uses[op] > 1 && applies_share_memory(op)) alone[k] = 1;
   std::vector<Sys<T>> sys(count);
   std::vector<Chunk> chunks;
   unsigned char* a = static_cast<unsigned char*>(s->arena);
@@ -434,7 +447,7 @@ int solve_wave(dgop_batch_solver* s, const std::vector<int>& wave, const double*
   const unsigned sysb = (unsigned)((count + kBT - 1) / kBT);
 
   auto residual = [&](int phase, cudaStream_t q) -> int {
-    DGOP_TRY_BS(per_system(s, count, q, [&](int k, cudaStream_t b) {
+    DGOP_TRY_BS(per_system(s, alone, q, [&](int k, cudaStream_t b) {
       return launch_f64(s->ops[wave[k]], 1.0, sys[k].x, 0.0, sys[k].w64, 0, b, &sys[k].st->done);
     }));
     kb_sub_norm<T><<<nch, kBT, 0, q>>>(dsys, s->d_chunks, s->part, pw);
@@ -446,7 +459,7 @@ int solve_wave(dgop_batch_solver* s, const std::vector<int>& wave, const double*
     kb_cycle_start<T><<<sysb, kBT, 0, q>>>(dsys, count, m);
     kb_scale_v0<T><<<nch, kBT, 0, q>>>(dsys, s->d_chunks);
     for (int j = 0; j < m; ++j) {
-      DGOP_TRY_BS(per_system(s, count, q, [&](int k, cudaStream_t b) {
+      DGOP_TRY_BS(per_system(s, alone, q, [&](int k, cudaStream_t b) {
         const int i = wave[k];
         const int* skip = &sys[k].st->inactive;
         T* vj = sys[k].V + (int64_t)j * sys[k].ld;
@@ -467,7 +480,7 @@ int solve_wave(dgop_batch_solver* s, const std::vector<int>& wave, const double*
     if (s->precs[wave[0]]) {
       // x += P (sum y_i V_i) (every system has a preconditioner: dgop_batch_solver_create)
       kb_update<T><<<nch, kBT, 0, q>>>(dsys, s->d_chunks, 0);
-      DGOP_TRY_BS(per_system(s, count, q, [&](int k, cudaStream_t b) {
+      DGOP_TRY_BS(per_system(s, alone, q, [&](int k, cudaStream_t b) {
         return launch_f64(s->precs[wave[k]], 1.0, sys[k].pt, 1.0, sys[k].x, 0, b, &sys[k].st->done);
       }));
     } else {

@@ -154,7 +154,8 @@ namespace dgop {
 // workspace (elements too large for shared memory), or the face words that a bulk-tensor launch
 // rebuilds from per-element velocity factors.  Such applies must not run at the same time.
 inline bool applies_share_memory(const dgop_operator* op) {
-  return op->f64.d_scratch != nullptr || (op->k64.factors && op->k64.d_tma != nullptr);
+  return op->f64.d_scratch != nullptr || op->f32.d_scratch != nullptr ||
+         (op->k64.factors && op->k64.d_tma != nullptr);
 }
 }  // namespace dgop
 

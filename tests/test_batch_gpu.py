@@ -286,3 +286,22 @@ def test_split_variant_groups(D, p, count, n):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(want, ys))
     batch.close()
+
+
+@pytest.mark.parametrize("inner", ["fp32", "fp64"])
+def test_batch_solver_with_a_repeated_operator_that_owns_a_workspace(inner):
+    """Several right-hand sides of one operator whose applies share a global workspace (see the batched
+    apply's test), beside another system: every system as when solved by itself (cut off after 40
+    steps, with the residual reached by then)."""
+    op = g.SystemOperator(_space(6, [2, 1, 2, 2, 1, 2], 2, g.GL), 4, C.velocity_constant([0.3, -0.2, 0.5, 0.1, -0.4, 0.2]),
+                          sigma=1e3)
+    assert op.kernel == "generic"
+    other = g.SystemOperator(_space(3, [5, 4, 3], 3), 5, C.velocity_constant([0.5, -0.2, 0.1]), sigma=1e3)
+    ops = [op, other, op, op, op]
+    bs = [torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops]
+    xs = [torch.zeros_like(b) for b in bs]
+    res, _ = g.BatchSolver(ops, None, restart=10, inner=inner).solve(bs, xs, 40, 1e-10)
+    for o, b, x, r in zip(ops, bs, xs, res):
+        alone = torch.zeros_like(b)
+        (one,), _ = g.BatchSolver([o], None, restart=10, inner=inner).solve([b], [alone], 40, 1e-10)
+        assert one == r and torch.equal(alone, x)
