@@ -350,7 +350,7 @@ class _Operator:
 
     def variant_times(self):
         """Autotuner time per launch (ms) of every variant (0.0: not available or not timed; the
-        any-dimension kernel's variants are timed on the first 16,384 elements)."""
+        any-dimension kernel's variants are timed on the first 65,536 elements)."""
         out = {}
         for k, name in enumerate(self._variants()):
             ms = ctypes.c_float()
@@ -574,10 +574,11 @@ class GMRESIRSolver(_Solver):
 
 
 class Batch:
-    """Independent operators applied together: one persistent launch per (dimension, order,
-    variant) group of any-dimension Kronecker operators, one launch each for the rest (other
-    kernels, variants without a persistent form, operators that fill the GPU on their own)
-    (dgop_batch_apply)."""
+    """Independent operators applied together (dgop_batch_apply): one persistent launch per (dimension,
+    order, variant) group of any-dimension Kronecker operators, one launch each for the rest (other
+    kernels, variants without a persistent form, operators large enough to fill the GPU or too few to
+    gain from a group), the launches spread over a few streams.  Applies of one batch may come on any
+    streams and threads."""
 
     def __init__(self, ops):
         self.ops = list(ops)

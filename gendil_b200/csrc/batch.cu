@@ -6,8 +6,8 @@
 // element batch of every operator of the group.  Operators on another kernel are applied one
 // launch each.  The launches are independent, so they are spread over the caller's stream and a
 // few more that fork from it and join it again (largest operators first): a launch's tail, and the
-// small operators, run beside the others (24 systems of 2D to 4D, p = 1..5: 213 us, 332 us in one
-// stream).  Results equal those of the operators' own applies bit for bit (same arithmetic).
+// small operators, run beside the others (24 systems of 2D to 4D, p = 1..5: 216 us, 332 us in one
+// stream).  Members that repeat an operator whose applies share device memory keep one stream.  Results equal those of the operators' own applies bit for bit (same arithmetic).
 #include <cuda_runtime.h>
 
 #include <algorithm>

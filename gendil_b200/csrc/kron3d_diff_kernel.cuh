@@ -8,7 +8,7 @@
 //   y = Mz [ My (Ax u + x faces) + Mx (Ay u + y faces) ]   layout Z, one exchange, one z pass
 //     + Az (My Mx u) + z faces                              layout Z, one exchange, one z pass
 //
-// Seven N x N passes and two exchanges.  A face's own terms are linear in the element's diffusivity
+// Eight N x N passes and two exchanges.  A face's own terms are linear in the element's diffusivity
 // mu_e and go into the pass: A_a = mu_e Kint_a with
 //   Kint_a = Khat_a + f sum_s ( -nu/2 b d^T + kappa/2 b b^T + sigma nu/2 d b^T ),  b = l(s), d = l'(s),
 // plus f kappa/2 mu_nb b b^T per interior side (on a slice for a basis with nodes on the faces).  What

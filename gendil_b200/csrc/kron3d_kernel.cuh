@@ -23,9 +23,10 @@
 // there, and results leave through the same buffer with coalesced stores.  Which traces an element
 // needs is one 32-bit face word per element, built at operator creation (kron_face_words); with
 // per-element velocity factors, which the caller may change between applies, the word is built
-// in the kernel.  Constant 1D matrices are read from kernel-parameter space, only
-// element-dependent ones from global memory.  For even N the layout exchanges can be register
-// butterflies (shfl_xor within the element's lanes); otherwise they go through a shared tile.
+// in the kernel (N <= 4 outside the general form: kron3d_p3_kernel.cuh instead).  Constant 1D matrices
+// are read from kernel-parameter space, only element-dependent ones from global memory.  For N = 2 and
+// 4 the layout exchanges can be register butterflies (shfl_xor within the element's lanes); otherwise
+// they go through a shared tile.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -422,7 +423,7 @@ __device__ __forceinline__ void scale_plane(Real f, Real (&X)[N][N]) {
 }
 
 // Layout exchange between the N lanes of an element: X[i][j] held by lane t (plane index t of
-// the third axis) becomes Y[i][k] = X_k[i][t].  Even N: shfl_xor butterflies on the lane bits;
+// the third axis) becomes Y[i][k] = X_k[i][t].  N = 2 and 4: shfl_xor butterflies on the lane bits;
 // at the stage on bit b each lane keeps the column of each pair (j, j|m) whose bit b matches its
 // own and trades the other with lane t ^ m.
 template <int N, typename Real>
@@ -831,7 +832,7 @@ constexpr int kron_max_warps = 4;  // warps per CTA of kron3d_kernel (128 thread
 // Kernel variants (chosen per operator by the autotuner):
 //   STAGES 2: the next group is staged while this one computes; 1: no overlap inside the warp,
 //   less shared memory per warp and so more warps per SM
-//   SHFL:    layout exchanges by shuffle butterflies (even N) instead of the shared tile
+//   SHFL:    layout exchanges by shuffle butterflies (N = 2, 4) instead of the shared tile
 //   DOT:     the inner-product epilogue (P.dot_partials; FP64 solvers) is compiled in
 //   VM:      the slot mask the kernel is compiled for (kVaryRuntime: read P.vary)
 //   GEN:     the general form: with P.gl a basis without nodes on the faces (the neighbours' traces

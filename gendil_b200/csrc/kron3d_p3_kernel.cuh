@@ -106,7 +106,7 @@ __device__ __forceinline__ bool p3_x_in_group(int s, int le, int ne, uint32_t cx
 }
 
 // Face terms of axis a added to a D-pass output Pm (plane [first][second]; the face slice is along
-// the first index when FIRST), from the element's face record (see stage_group).  nbrow(side, src,
+// the first index when FIRST), from the element's face record (see p3_stage_group).  nbrow(side, src,
 // e_nb, v) reads this lane's row of the neighbour trace of that side from the group's staged DoFs
 // (x only), the axis' staged trace slot (V-wide), or global memory.
 template <int N, typename Real, bool FIRST, typename NbRow>

@@ -228,7 +228,7 @@ KronPlanHost plan_kron3d(const KronInputs& in) {
     p.why = "dimension != 3";
     return p;
   }
-  if (in.N > kKronMaxN) {  // the FP64 register kernel spills above N = 6
+  if (in.N > kKronMaxN) {  // FP64 at N = 6 is at the register limit (254 and up, 4 to 216 bytes spilled)
     p.why = "order above 5 (register kernel limit)";
     return p;
   }
