@@ -266,7 +266,12 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
         set_error("dgop_batch_apply: null or aliasing vectors");
         return DGOP_ERR_ARG;
       }
-  if (!b->groups.empty()) {
+  // Under stream capture the groups' members are launched one by one (the same results): a table upload in the
+  // graph would read whatever the staging buffer holds when the graph runs.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+  const bool grouped = capture == cudaStreamCaptureStatusNone && !b->groups.empty();
+  if (grouped) {
     // the staging buffer of the previous apply may still be in flight
     DGOP_CUDA_B(cudaEventSynchronize(b->uploaded));
     for (auto& g : b->groups)
@@ -302,7 +307,12 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     rc = dgop_apply(b->ops[i], x[i], y[i], stream_of());
   }
   for (auto& g : b->groups) {
-    if (rc != DGOP_OK) break;
+    if (!grouped)
+      for (size_t k = 0; rc == DGOP_OK && k < g.members.size(); ++k) {
+        const size_t lane = k % (ns + 1);
+        rc = dgop_apply(b->ops[g.members[k]], x[g.members[k]], y[g.members[k]], lane ? b->side[lane - 1] : st);
+      }
+    if (rc != DGOP_OK || !grouped) continue;
     g.entry->launch_batch[g.variant](g.d_table, g.d_first, (int)g.members.size(), g.eb, g.grid, g.block, g.smem,
                                      stream_of());
     keep(cudaGetLastError(), "batch kernel launch");
@@ -311,7 +321,7 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
   for (size_t k = 0; k < forked; ++k)
     if (keep(cudaEventRecord(b->joined[k], b->side[k]), "batch join"))
       keep(cudaStreamWaitEvent(st, b->joined[k], 0), "batch join");
-  if (!b->groups.empty()) keep(cudaEventRecord(b->applied, st), "batch event");
+  if (grouped) keep(cudaEventRecord(b->applied, st), "batch event");
   return rc;
 }
 

@@ -181,7 +181,8 @@ int dgop_apply_f32(dgop_operator* op, const float* x, float* y, void* stream);
  * fork from it and join it; members that repeat an operator whose applies share device memory
  * run in turn.  y[i] = A_i x[i] (device pointers), bit-identical to dgop_apply.  The operators must
  * outlive the batch.  Applies of one batch may come from several threads and on several streams (the
- * kernels of one apply finish with the batch's tables before the next apply replaces them).
+ * kernels of one apply finish with the batch's tables before the next apply replaces them), and under
+ * stream capture, where every operator is launched on its own.
  * dgop_batch_groups gives the number of grouped launches. */
 typedef struct dgop_batch dgop_batch;
 int dgop_batch_create(dgop_operator* const* ops, int count, dgop_batch** out);

@@ -305,3 +305,35 @@ def test_batch_solver_with_a_repeated_operator_that_owns_a_workspace(inner):
         alone = torch.zeros_like(b)
         (one,), _ = g.BatchSolver([o], None, restart=10, inner=inner).solve([b], [alone], 40, 1e-10)
         assert one == r and torch.equal(alone, x)
+
+
+@pytest.mark.parametrize("specs", [[(3, 5, 3), (3, 6, 2), (3, 4, 4)],
+                                   [(2, 9, 1), (2, 11, 1), (4, 4, 2), (4, 3, 2), (4, 5, 2), (4, 3, 2), (3, 4, 3)]],
+                         ids=["single_launches", "groups"])
+def test_batch_under_stream_capture(specs):
+    """A captured batched apply replays with the vectors it was captured with, whatever the batch did
+    in between, and the batch applies eagerly before and after."""
+    rng = np.random.default_rng(8)
+    ops = []
+    for D, n, p in specs:
+        o = g.SystemOperator(_space(D, n, p), p + 2, C.velocity_constant(list(rng.uniform(-1, 1, D))), sigma=1e3)
+        if D % 2 == 0:
+            o.set_variant("nd-split")
+        ops.append(o)
+    batch = g.Batch(ops)
+    assert batch.groups == (2 if len(specs) > 3 else 0)
+    xs = [torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops]
+    ys, other = [torch.zeros_like(x) for x in xs], [torch.zeros_like(x) for x in xs]
+    batch.apply(xs, other)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        batch.apply(xs, ys)
+    for _ in range(2):
+        for x in xs:
+            x.mul_(-0.5)
+        want = [o(x, torch.empty_like(x)) for o, x in zip(ops, xs)]
+        batch.apply([w.clone() for w in want], other)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for y, w in zip(ys, want))
