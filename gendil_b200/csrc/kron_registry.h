@@ -35,7 +35,7 @@ struct KronVariant {
   // compile-time slot-mask forms of the above (one-stage tile variants): [mask index, kron.h]
   // [with the inner-product epilogue][separate mass term]
   const void* func_masked[2][2][2] = {};
-  // the general form (KronParams::general): [with the inner-product epilogue][separate mass term]
+  // the general form (KronHead::general): [with the inner-product epilogue][separate mass term]
   const void* func_general[2][2] = {};
   // the forms for per-element velocity factors (kron_early_factors): [with the inner-product epilogue]
   // [separate mass term][0: run-time slot mask, mask index + 1]
@@ -57,7 +57,8 @@ struct KronEntry {
                       cudaStream_t s) = nullptr;
   const void* func_diff[2][3] = {};
   int diff_warp_smem[2] = {};
-  // face words of the forward and the transposed operator (KronParams::eflags), 2 nelem of them; the bulk-tensor variants' face and slot words
+  // face words of the forward and the transposed operator (KronHead::eflags), 2 nelem of them; the
+  // bulk-tensor variants' face and slot words
   void (*face_words)(const KronParams<Real>& fwd, const KronParams<Real>& tr, uint32_t* words, cudaStream_t s) = nullptr;
   void (*tma_words)(const KronParams<Real>& p, uint32_t* eflags, uint32_t* gwords, cudaStream_t s) = nullptr;
 };
