@@ -35,13 +35,26 @@ struct BatchGroup {
   size_t smem = 0;
   dim3 grid, block;
 };
+// Small 3D register-kernel operators of one order in one launch (kron3d_pack_kernel).
+struct BatchPack {
+  const KronVariant<double>* variant = nullptr;
+  std::vector<int> members;
+  bool sep = false;                 // with a separate mass term
+  std::vector<double> parameters;   // of the launch (KronVariant::fill_pack); x and y set per apply
+  dim3 grid, block;
+  size_t smem = 0;
+  KronHead<double>& head(size_t k) {
+    return *reinterpret_cast<KronHead<double>*>(reinterpret_cast<unsigned char*>(parameters.data()) + k * variant->pack_stride);
+  }
+};
 }  // namespace
 
 struct dgop_batch {
   std::vector<dgop_operator*> ops;
   std::vector<BatchGroup> groups;
+  std::vector<BatchPack> packs;
   std::vector<int> singles;  // operators applied one launch each
-  std::vector<size_t> lane;  // stream of every launch, the singles' then the groups' (0: the caller's)
+  std::vector<size_t> lane;  // stream of every launch: the singles', the groups', the packs' (0: the caller's)
   cudaEvent_t uploaded = nullptr;  // the staging buffer has been read
   cudaEvent_t applied = nullptr;   // the last apply's launches are done with the device tables
   std::mutex mutex;                // an apply's events and staging are one thread's at a time
@@ -153,6 +166,63 @@ int setup(dgop_batch* b) {
       ++k;
     }
   }
+  // Small 3D register-kernel operators above p = 3: several in one launch, under the split variant's rules.
+  // A launch of 30 KB of parameters costs the host 7 to 17 us, seven or ten launches of one operator 5 us each (us,
+  // one launch each / together: 64 systems of p = 4, 14,000 dofs 347 / 247, 129,000 dofs 345 / 190; of p = 5, 25,000
+  // dofs 336 / 196; 512 of p = 4, 135,000 dofs 2621 / 1502).
+  std::map<std::pair<int, bool>, std::vector<int>> small;
+  for (size_t k = 0; k < b->singles.size();) {
+    const int i = b->singles[k];
+    const dgop_operator* op = b->ops[i];
+    const auto& K = op->k64;
+    if (op->kernel == DGOP_KERNEL_KRON && K.ready && K.entry->v[K.variant].launch_pack && !K.params.general &&
+        !K.factors && op->sp.ndofs <= kSplitGroupDofs && mean <= kSplitMeanDofs) {
+      const auto& p = K.params;
+      small[{op->sp.n, p.has_adv && p.has_mass && !p.mass_merged}].push_back(i);
+      b->singles.erase(b->singles.begin() + (long)k);
+    } else {
+      ++k;
+    }
+  }
+  for (const auto& [key, members] : small) {
+    if (members.size() < kSplitGroupMembers) {
+      b->singles.insert(b->singles.end(), members.begin(), members.end());
+      continue;
+    }
+    for (size_t m = 0; m < members.size();) {
+      BatchPack pack;
+      const auto& K0 = b->ops[members[m]]->k64;
+      pack.variant = &K0.entry->v[K0.variant];
+      const auto& L = K0.launch[K0.variant];
+      pack.block = L.block;
+      pack.smem = L.smem;
+      const void* fn = pack.variant->func_pack[key.second ? 1 : 0];
+      cudaFuncAttributes fa{};
+      DGOP_CUDA_B(cudaFuncGetAttributes(&fa, fn));
+      DGOP_CUDA_B(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)fa.sharedSizeBytes));
+      unsigned blocks = 1;
+      for (; m < members.size() && (int)pack.members.size() < pack.variant->pack; ++m) {
+        pack.members.push_back(members[m]);
+        blocks = std::max(blocks, b->ops[members[m]]->k64.launch[K0.variant].grid.x);
+      }
+      pack.grid = dim3(blocks, (unsigned)pack.members.size());
+      pack.sep = key.second;
+      pack.parameters.resize((pack.variant->pack_bytes + sizeof(double) - 1) / sizeof(double));
+      std::vector<KronParams<double>> params;
+      for (int i : pack.members) {
+        params.push_back(b->ops[i]->k64.params);
+        params.back().alpha = 1.0;
+        params.back().beta_y = 0.0;
+        params.back().flags = b->ops[i]->flags;
+        params.back().e_begin = 0;
+        params.back().nelem = b->ops[i]->sp.nelem;
+      }
+      std::vector<const KronParams<double>*> at;
+      for (const auto& p : params) at.push_back(&p);
+      pack.variant->fill_pack(at.data(), (int)at.size(), pack.parameters.data());
+      b->packs.push_back(std::move(pack));
+    }
+  }
   for (auto& g : b->groups) {
     g.first.push_back(0);
     for (int i : g.members) {
@@ -190,7 +260,7 @@ int setup(dgop_batch* b) {
   constexpr size_t kStreams = 6;
   std::stable_sort(b->singles.begin(), b->singles.end(),
                    [&](int i, int j) { return b->ops[i]->sp.ndofs > b->ops[j]->sp.ndofs; });
-  const size_t launches = b->groups.size() + b->singles.size();
+  const size_t launches = b->groups.size() + b->singles.size() + b->packs.size();
   for (size_t k = 1; k < std::min(launches, kStreams); ++k) {
     cudaStream_t s = nullptr;
     DGOP_CUDA_B(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -251,7 +321,7 @@ int dgop_batch_create(dgop_operator* const* ops, int count, dgop_batch** out) {
   return DGOP_OK;
 }
 
-int dgop_batch_groups(const dgop_batch* b) { return b ? (int)b->groups.size() : -1; }
+int dgop_batch_groups(const dgop_batch* b) { return b ? (int)(b->groups.size() + b->packs.size()) : -1; }
 
 int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, void* stream) {
   if (!b || !x || !y) {
@@ -316,6 +386,26 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     g.entry->launch_batch[g.variant](g.d_table, g.d_first, (int)g.members.size(), g.eb, g.grid, g.block, g.smem,
                                      stream_of());
     keep(cudaGetLastError(), "batch kernel launch");
+  }
+  if (!grouped) next = b->singles.size() + b->groups.size();
+  for (auto& g : b->packs) {
+    if (rc != DGOP_OK) break;
+    const cudaStream_t q = stream_of();
+    bool together = true;
+    for (size_t k = 0; k < g.members.size(); ++k) {
+      const int i = g.members[k];
+      const uintptr_t ax = reinterpret_cast<uintptr_t>(x[i]), ay = reinterpret_cast<uintptr_t>(y[i]);
+      together = together && ax && ay && ax != ay && ax % 16 == 0 && ay % 16 == 0;
+      g.head(k).x = x[i];
+      g.head(k).y = y[i];
+    }
+    if (together) {
+      g.variant->launch_pack(g.parameters.data(), g.sep, g.grid, g.block, g.smem, q);
+      keep(cudaGetLastError(), "batch kernel launch");
+    } else {  // vectors off 16 bytes take another kernel, others are errors: each by its own apply
+      for (size_t k = 0; rc == DGOP_OK && k < g.members.size(); ++k)
+        rc = dgop_apply(b->ops[g.members[k]], x[g.members[k]], y[g.members[k]], q);
+    }
   }
   // join every forked stream, also after an error: the caller's stream waits for what was queued
   for (size_t k = 0; k < forked; ++k)

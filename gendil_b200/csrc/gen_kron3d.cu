@@ -116,6 +116,17 @@ void fill_fact(KronVariant<Real>& v) {
   }
 }
 
+template <int N>
+void fill_pack(const KronParams<double>* const* p, int count, void* block) {
+  for (int i = 0; i < count; ++i) static_cast<KronPack<N>*>(block)->p[i] = kron_block<N, false>(*p[i]);
+}
+template <int N>
+void launch_pack(const void* block, bool sep, dim3 grid, dim3 threads, size_t smem, cudaStream_t s) {
+  const KronPack<N>& a = *static_cast<const KronPack<N>*>(block);
+  if (sep) kron3d_pack_kernel<N, true><<<grid, threads, smem, s>>>(a);
+  else kron3d_pack_kernel<N, false><<<grid, threads, smem, s>>>(a);
+}
+
 template <int N, typename Real, int STAGES, bool SHFL>
 void fill_variant(KronVariant<Real>& v) {
   v.launch = &launch_kron3d<N, Real, STAGES, SHFL>;
@@ -243,6 +254,15 @@ void fill(KronEntry<Real>& d) {
   // above p = 3 one staging stage: two of them and the exchange tile leave too few warps per SM
   if constexpr (N <= 4) fill_variant<N, Real, 2, false>(d.v[0]);
   fill_variant<N, Real, 1, false>(d.v[1]);
+  if constexpr (N > 4 && std::is_same<Real, double>::value) {
+    d.v[1].fill_pack = &fill_pack<N>;
+    d.v[1].launch_pack = &launch_pack<N>;
+    d.v[1].pack_bytes = sizeof(KronPack<N>);
+    d.v[1].pack_stride = sizeof(KronParams<double, N, false>);
+    d.v[1].func_pack[0] = reinterpret_cast<const void*>(&kron3d_pack_kernel<N, false>);
+    d.v[1].func_pack[1] = reinterpret_cast<const void*>(&kron3d_pack_kernel<N, true>);
+    d.v[1].pack = KronPack<N>::MAX;
+  }
   if constexpr (Kron3DShape<N, Real>::BUTTERFLY) fill_variant<N, Real, 2, true>(d.v[2]);
   d.face_words = &face_words<Real>;
   if constexpr (N >= 2) {

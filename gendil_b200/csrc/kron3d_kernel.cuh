@@ -1128,6 +1128,20 @@ __global__ void __launch_bounds__(128, kron3d_min_ctas<N, Real>())
   kron3d_body<N, Real, SEP, STAGES, SHFL, DOT, VM, GEN>(P);
 }
 
+// Several small operators of one order in one launch (above p = 3): instance blockIdx.y's parameters are an
+// entry of the launch's own parameters, so nothing has to be uploaded.  As many as a launch takes (32,764 bytes):
+// 10 at N = 5, 7 at N = 6.  Same arithmetic as each operator's own launch (batch.cu says when it pays).
+template <int N>
+struct KronPack {
+  static constexpr int MAX = 32000 / (int)sizeof(KronParams<double, N, false>);
+  KronParams<double, N, false> p[MAX];
+};
+template <int N, bool SEP>
+__global__ void __launch_bounds__(128, kron3d_min_ctas<N, double>())
+    kron3d_pack_kernel(const __grid_constant__ KronPack<N> A) {
+  kron3d_body<N, double, SEP, 1, false, false, kVaryRuntime, false>(A.p[blockIdx.y]);
+}
+
 // Face words of every element (P.eflags of later launches), for operators with advection terms:
 // words[e] of the forward operator, words[nelem + e] of the transposed one.
 template <typename Real>

@@ -40,6 +40,14 @@ struct KronVariant {
   // the forms for per-element velocity factors (kron_early_factors): [with the inner-product epilogue]
   // [separate mass term][0: run-time slot mask, mask index + 1]
   const void* func_fact[2][2][3] = {};
+  // several operators in one launch (FP64, above p = 3): fill_pack writes the parameters of `count` <= pack of
+  // them, all or none with a separate mass term, to a block of pack_bytes whose instance k's KronHead is at
+  // k * pack_stride; launch_pack launches that block, grid.x covering the largest, grid.y = count
+  void (*fill_pack)(const KronParams<Real>* const* p, int count, void* block) = nullptr;
+  void (*launch_pack)(const void* block, bool sep, dim3 grid, dim3 threads, size_t smem, cudaStream_t s) = nullptr;
+  const void* func_pack[2] = {};   // [separate mass term]
+  int pack = 0;
+  size_t pack_bytes = 0, pack_stride = 0;
   int warp_smem = 0;               // Real values of shared memory per warp (bytes per CTA for bulk-tensor variants)
   int warp_smem_general = 0;       // Real values per warp of the general form
   int warp_smem_fact = 0;          // and of the forms for velocity factors

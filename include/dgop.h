@@ -175,9 +175,9 @@ int dgop_apply_f32(dgop_operator* op, const float* x, float* y, void* stream);
 /* Batches of independent operators (no reference counterpart; configuration 5 of the benchmark
  * plan): operators on the any-dimension Kronecker kernel are grouped by (dimension, order, kernel
  * variant) and each group is applied by ONE persistent launch over all its operators' elements;
- * the others (other kernels, such as the 3D register kernel, variants without a persistent form,
- * operators large enough to fill the GPU, and few or large operators of the split variant) are
- * applied one launch each.  The launches are independent, on the caller's stream and a few that
+ * small 3D operators on the register kernel above order 3 share launches too; the others (other
+ * kernels, variants without a persistent form, operators large enough to fill the GPU, and few or
+ * large operators of the split variant and above order 3) are applied one launch each.  The launches are independent, on the caller's stream and a few that
  * fork from it and join it; members that repeat an operator whose applies share device memory
  * run in turn.  y[i] = A_i x[i] (device pointers), bit-identical to dgop_apply.  The operators must
  * outlive the batch.  Applies of one batch may come from several threads and on several streams (the

@@ -337,3 +337,35 @@ def test_batch_under_stream_capture(specs):
         graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(y, w) for y, w in zip(ys, want))
+
+
+@pytest.mark.parametrize("p", [4, 5])
+def test_small_3d_operators_above_order_3_share_launches(p):
+    """More operators than one launch takes, of both term structures, from one element to several CTAs,
+    velocities constant and varying, periodic and not: bit for bit their own applies, also with one vector
+    off 16 bytes (whose launch falls back to single applies)."""
+    rng = np.random.default_rng(p)
+    ops = []
+    for i in range(24):
+        sizes = [1 + i % 5, 1 + i % 3, 1 + i % 4] if i else [9, 8, 7]
+        sp = g.Space(3, sizes, [1.0 / n for n in sizes], None, [i % 2, 0, (i // 2) % 2], p)
+        beta = C.velocity_sincos(3) if i % 4 == 1 else C.velocity_constant(list(rng.uniform(-1, 1, 3)))
+        sigma = C.Coefficient(terms=[{0: lambda x: 1 + x}]) if i >= 12 else 1e3
+        ops.append(g.SystemOperator(sp, p + 2, beta, sigma=sigma, bc=g.BC_INFLOW, g=0.3))
+        assert ops[-1].kernel == "kron", ops[-1].kernel_note
+    xs = [torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops]
+    want = [o(x, torch.empty_like(x)) for o, x in zip(ops, xs)]
+    batch = g.Batch(ops)
+    assert 2 <= batch.groups <= 6
+    for off in (None, 3):
+        ys = [torch.full_like(x, float("nan")) for x in xs]
+        if off is not None:
+            ys[off] = torch.full((xs[off].numel() + 1,), float("nan"), dtype=torch.float64, device="cuda")[1:]
+        batch.apply(xs, ys)
+        torch.cuda.synchronize()
+        for k, (y, w) in enumerate(zip(ys, want)):
+            if k == off:  # the any-dimension kernel
+                assert float((y - w).abs().max()) <= 1e-13 * float(w.abs().max())
+            else:
+                assert torch.equal(y, w), k
+    batch.close()
