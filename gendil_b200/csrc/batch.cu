@@ -51,6 +51,7 @@ struct BatchPack {
 
 struct dgop_batch {
   std::vector<dgop_operator*> ops;
+  std::vector<int> versions;  // of the operators' launch configurations, when the batch was made
   std::vector<BatchGroup> groups;
   std::vector<BatchPack> packs;
   std::vector<int> singles;  // operators applied one launch each
@@ -310,6 +311,7 @@ int dgop_batch_create(dgop_operator* const* ops, int count, dgop_batch** out) {
       return DGOP_ERR_ARG;
     }
     b->ops.push_back(ops[i]);
+    b->versions.push_back(ops[i]->version);
   }
   const int rc = setup(b);
   if (rc != DGOP_OK) {
@@ -376,22 +378,33 @@ int dgop_batch_apply(dgop_batch* b, const double* const* x, double* const* y, vo
     if (rc != DGOP_OK) break;
     rc = dgop_apply(b->ops[i], x[i], y[i], stream_of());
   }
+  // members whose kernel or variant was chosen anew since the batch was made apply on their own
+  auto as_made = [&](const std::vector<int>& members) {
+    for (int i : members)
+      if (b->ops[i]->version != b->versions[i]) return false;
+    return true;
+  };
   for (auto& g : b->groups) {
-    if (!grouped)
+    const bool one_launch = grouped && as_made(g.members);
+    if (!one_launch)
       for (size_t k = 0; rc == DGOP_OK && k < g.members.size(); ++k) {
-        const size_t lane = k % (ns + 1);
-        rc = dgop_apply(b->ops[g.members[k]], x[g.members[k]], y[g.members[k]], lane ? b->side[lane - 1] : st);
+        dgop_operator* op = b->ops[g.members[k]];
+        const size_t lane = applies_share_memory(op) ? 0 : k % (ns + 1);
+        rc = dgop_apply(op, x[g.members[k]], y[g.members[k]], lane ? b->side[lane - 1] : st);
       }
-    if (rc != DGOP_OK || !grouped) continue;
+    if (!one_launch) {
+      ++next;
+      continue;
+    }
+    if (rc != DGOP_OK) break;
     g.entry->launch_batch[g.variant](g.d_table, g.d_first, (int)g.members.size(), g.eb, g.grid, g.block, g.smem,
                                      stream_of());
     keep(cudaGetLastError(), "batch kernel launch");
   }
-  if (!grouped) next = b->singles.size() + b->groups.size();
   for (auto& g : b->packs) {
     if (rc != DGOP_OK) break;
     const cudaStream_t q = stream_of();
-    bool together = true;
+    bool together = as_made(g.members);
     for (size_t k = 0; k < g.members.size(); ++k) {
       const int i = g.members[k];
       const uintptr_t ax = reinterpret_cast<uintptr_t>(x[i]), ay = reinterpret_cast<uintptr_t>(y[i]);

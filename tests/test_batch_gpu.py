@@ -369,3 +369,23 @@ def test_small_3d_operators_above_order_3_share_launches(p):
             else:
                 assert torch.equal(y, w), k
     batch.close()
+
+
+def test_batch_follows_a_kernel_chosen_after_it_was_made():
+    """Operators of a group, and of a shared launch, whose kernel is chosen anew after the batch was made are
+    applied as their own applies are."""
+    ops = [g.SystemOperator(_space(2, n, 2), 4, C.velocity_constant([0.3, -0.4]), sigma=1e3) for n in (9, 11, 7, 8)]
+    for o in ops:
+        o.set_variant("nd-split")
+    ops += [g.SystemOperator(_space(3, n, 4), 6, C.velocity_constant([0.3, -0.4, 0.2]), sigma=1e3) for n in (3, 4, 2, 3)]
+    xs = [torch.rand(o.space.num_dofs, dtype=torch.float64, device="cuda") - 0.5 for o in ops]
+    batch = g.Batch(ops)
+    assert batch.groups == 2
+    for change in (None, 0, 4):
+        if change is not None:
+            ops[change].select_kernel("generic")
+        want = [o(x, torch.empty_like(x)) for o, x in zip(ops, xs)]
+        ys = [torch.full_like(x, float("nan")) for x in xs]
+        batch.apply(xs, ys)
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for y, w in zip(ys, want)), change
